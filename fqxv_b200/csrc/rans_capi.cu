@@ -306,10 +306,10 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
         // 32 per byte; the batch's throughput time is the sum over streams
         // of bytes x (SM cycles per byte at the class's full-GPU rate) / SMs.
         auto lat_cpb = [](const DecStream &d) {
-            return d.cls == kClsO0 ? 5.0 : d.nd <= kShflMaxNd ? 15.0 : d.nd <= kSmallMaxNd ? 18.0 : 19.5;
+            return d.cls == kClsO0 ? 5.0 : d.nd <= kTinyMaxNd ? 8.0 : d.nd <= kMidMaxNd ? 11.0 : 19.5;
         };
         auto rate_cpb = [](const DecStream &d) {
-            return d.cls == kClsO0 ? 0.9 : d.cls == kClsO1Global ? 14.0 : d.nd <= kSmallMaxNd ? 3.0 : 7.0;
+            return d.cls == kClsO0 ? 0.9 : d.cls == kClsO1Global ? 14.0 : d.nd <= kTinyMaxNd ? 1.5 : d.nd <= kMidMaxNd ? 2.5 : 7.0;
         };
         double bulk = 0;
         for (size_t i = 0; i < nb; i++)
@@ -333,7 +333,8 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
             if (d.cls == kClsO0) return 0;
             if (d.cls == kClsO1Global) return kGroups - 1;
             if (d.cls != kClsO1Dense) return -1;
-            if (d.nd <= kSmallMaxNd) return is_top[i] ? kGroupSmallTop : 1;
+            if (d.nd <= kTinyMaxNd) return is_top[i] ? kGroupTinyTop : kGroupTiny;
+            if (d.nd <= kMidMaxNd) return is_top[i] ? kGroupMidTop : kGroupMid;
             if (is_top[i]) return kGroupFourTop;
             return d.tbl_bytes <= (uint64_t)ctx->tune.dense_edge_small   ? kGroupDense0
                    : d.tbl_bytes <= (uint64_t)ctx->tune.dense_edge_large ? kGroupDense0 + 1
@@ -360,16 +361,17 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
         for (int g = 0; g < kGroups; g++) {
             if (g == 0) gcls[g] = kClsO0;
             else if (g == kGroups - 1) gcls[g] = kClsO1Global;
-            else if (g == 1 || g == kGroupSmallTop) gcls[g] = kClsO1Small;
+            else if (g == kGroupTiny || g == kGroupTinyTop) gcls[g] = kClsO1Small;
+            else if (g == kGroupMid || g == kGroupMidTop) gcls[g] = kClsO1Mid;
             else if (g == kGroupFourTop) gcls[g] = kClsO1Dense;
             else gcls[g] = (int64_t)lists[g].size() < four_max ? kClsO1Dense : kClsO1Wide;
             // the four-warp decoder also stages the bit-plane columns
             smem[g] = dec_smem_bytes(gcls[g], gcls[g] == kClsO1Dense ? tmaxp[g] : tmax[g], ndmax[g]);
             // the groups of largest streams: one CTA per SM, alone on it
-            if ((g == kGroupFourTop || g == kGroupSmallTop) && ctx->tune.o1_top_exclusive)
-                smem[g] = std::max(smem[g], dec_exclusive_smem(gcls[g], g == kGroupSmallTop
-                                                                              ? (int)ctx->tune.o1_top_small_per_sm
-                                                                              : 1));
+            if (is_top_group(g) && ctx->tune.o1_top_exclusive)
+                smem[g] = std::max(smem[g], dec_exclusive_smem(gcls[g], g == kGroupFourTop
+                                                                              ? 1
+                                                                              : (int)ctx->tune.o1_top_small_per_sm));
         }
         // Groups are launched longest first -- by the serial time of their
         // largest stream (rounds x cycles per round: ~620 for order-1,
@@ -390,6 +392,7 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
             at += lists[g].size();
         }
         if (tot) CK(cudaMemcpyAsync(ctx->d_order.p, hl, tot * 4, cudaMemcpyHostToDevice, s));
+        static_assert(4 * 4 * kGroups <= 512, "a queue head per group");
         CK(cudaMemsetAsync(queue, 0, 4 * 4 * kGroups, s));
         CK(cudaEventRecord(ctx->ev_fork, s));
         const uint32_t *dl = ctx->d_order.as<uint32_t>();
@@ -399,19 +402,20 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
             if (!m) continue;
             const int cls = gcls[g];
             const int stage = cls == kClsO0 ? kStDecO0 : cls == kClsO1Global ? kStDecO1Global
-                              : cls == kClsO1Small ? kStDecO1Small : cls == kClsO1Wide ? kStDecO1Wide
+                              : cls == kClsO1Small || cls == kClsO1Mid ? kStDecO1Small : cls == kClsO1Wide ? kStDecO1Wide
                                                                                          : kStDecO1Dense;
             cudaStream_t as = ctx->aux[g];
             CK(cudaStreamWaitEvent(as, ctx->ev_fork, 0));
             int per_sm = dec_blocks_per_sm(cls, smem[g]);
             const Tuning &T = ctx->tune;
-            int64_t cap = cls == kClsO0 ? T.cta_cap_o0 : cls == kClsO1Small ? T.cta_cap_o1_small
+            const bool small = cls == kClsO1Small || cls == kClsO1Mid;
+            int64_t cap = cls == kClsO0 ? T.cta_cap_o0 : small ? T.cta_cap_o1_small
                           : cls == kClsO1Wide ? T.cta_cap_o1_wide : cls == kClsO1Dense ? T.cta_cap_o1_four
                                                                                       : T.cta_cap_o1_global;
             // A batch bound by its top groups only needs the rest done by
             // then: fewer one-warp CTAs per SM slow its largest streams less.
-            if (ntop && g != kGroupSmallTop && g != kGroupFourTop) {
-                if (cls == kClsO1Small) cap = std::min<int64_t>(cap, T.cta_cap_o1_small_topped);
+            if (ntop && !is_top_group(g)) {
+                if (small) cap = std::min<int64_t>(cap, T.cta_cap_o1_small_topped);
                 if (cls == kClsO1Wide) cap = std::min<int64_t>(cap, T.cta_cap_o1_wide_topped);
             }
             per_sm = std::max(1, std::min<int>(per_sm, (int)cap));
@@ -576,7 +580,7 @@ int fqxv_rans_ctx_create(int device, fqxv_rans_ctx **out) {
     }
     for (int i = 0; i < kGroups && ok; i++)
         ok = cudaStreamCreateWithPriority(&c->aux[i], cudaStreamNonBlocking,
-                                          i == kGroupFourTop || i == kGroupSmallTop ? prio_hi : prio_lo) ==
+                                          is_top_group(i) ? prio_hi : prio_lo) ==
                  cudaSuccess &&
              cudaEventCreateWithFlags(&c->ev_join[i], cudaEventDisableTiming) == cudaSuccess;
     if (!ok) {

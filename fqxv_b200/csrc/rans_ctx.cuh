@@ -73,15 +73,20 @@ struct HostBuf {
     }
 };
 
-// Decode launch groups: order-0; order-1 small alphabets; order-1 wide
-// alphabets in three table-size ranges; the order-1 streams that bound the
-// batch by their serial time, wide alphabets (four-warp decoder) and small
-// ones, each group on SMs of its own; order-1 global tables.
-constexpr int kGroupDense0 = 2;   // first of the three dense table-size groups
+// Decode launch groups: order-0; order-1 tiny alphabets; order-1 alphabets of
+// up to kMidMaxNd symbols; order-1 wide alphabets in three table-size ranges;
+// the order-1 streams that bound the batch by their serial time, wide
+// alphabets (four-warp decoder), tiny ones and those between, each group on
+// SMs of its own; order-1 global tables.
+constexpr int kGroupTiny = 1;
+constexpr int kGroupMid = 2;
+constexpr int kGroupDense0 = 3;   // first of the three dense table-size groups
 constexpr int kDenseGroups = 3;
 constexpr int kGroupFourTop = kGroupDense0 + kDenseGroups;
-constexpr int kGroupSmallTop = kGroupFourTop + 1;
-constexpr int kGroups = kGroupSmallTop + 2;
+constexpr int kGroupTinyTop = kGroupFourTop + 1;
+constexpr int kGroupMidTop = kGroupTinyTop + 1;
+constexpr int kGroups = kGroupMidTop + 2;
+inline bool is_top_group(int g) { return g >= kGroupFourTop && g <= kGroupMidTop; }
 
 enum Stage {
     kStEncModel, kStEncRun, kStEncScan, kStEncPack, kStDecParse, kStDecO0, kStDecO1Dense, kStDecO1Global,
@@ -96,7 +101,7 @@ const char *const kStageNames[kStages] = {"enc_model", "enc_run", "enc_select_sc
 // library's run-time rules; a tuning table measured on the device replaces
 // them.
 struct Tuning {
-    // Order-1 streams of more than kSmallMaxNd symbols with shared-memory
+    // Order-1 streams of more than kMidMaxNd symbols with shared-memory
     // tables: a launch group of fewer than this many goes to the four-warp
     // decoder (one stream per SM), larger groups to the one-warp decoder
     // (several per SM). -1: the SM count.

@@ -95,15 +95,17 @@ struct DecStream {
 
 enum { kClsNone = 0, kClsO0 = 1, kClsO1Dense = 2, kClsO1Global = 3 };
 // Launch classes of dense streams decoded by one warp each: |D| <=
-// kSmallMaxNd (packed columns, chains stepped in registers) and wider
-// alphabets (byte columns, up to five chains per lane). kClsO1Dense is the
+// kTinyMaxNd (a column is one word, a chain step one rotate), |D| <=
+// kMidMaxNd (a byte column in four registers, a step two byte permutes) and
+// wider alphabets (a step is a shared-memory load). kClsO1Dense is the
 // four-warp decoder of the byte columns.
 constexpr int kClsO1Small = 4;
 constexpr int kClsO1Wide = 5;
-constexpr int kSmallMaxNd = 15;
-// Up to this |D| every chain of a round has its own lane (3 |D| + 1 <= 31)
-// and rows are resolved by shuffles; above it rows go through shared memory.
-constexpr int kShflMaxNd = 10;
+constexpr int kClsO1Mid = 6;
+// Six entries (|D| and DEAD) of five bits are what a 32-bit column holds.
+constexpr int kTinyMaxNd = 5;
+// 16 entries of a byte column fit in four registers.
+constexpr int kMidMaxNd = 15;
 
 // Decode table arena per stream (bytes from tbl_off).
 //   order-0: 4096 x u32 packed ((freq - 1) << 20) | ((slot - cum) << 8) | sym.
@@ -117,19 +119,24 @@ constexpr int kShflMaxNd = 10;
 //     [0, 4096)                 M8: u8 per slot, the slot's column less the
 //                               first column of its 256-slot block
 //     [4096, 4160)              MB: u32 per 256-slot block, that first
-//                               column (times S for byte columns: a byte
-//                               offset)
-//     [4160, + fc_bytes)        u32 (freq << 12) | cum, row = context, col = symbol
-//     [.., + 256)               dense index -> byte value
-//     [col_off, + ncol * S)     columns, S = dense_col_stride(nd) bytes each:
+//                               column times S (a byte offset)
+//     [4160, + fc_bytes)        u32 ((freq - 1) << 20) | (cum << 8) | byte,
+//                               row = context, col = symbol: one lookup gives
+//                               the step and the output byte
+//     [col_off, + (ncol + 1) S) columns, S = dense_col_stride(nd) bytes each:
 //                               byte d of column j = the dense symbol that
 //                               context d decodes in column j's slots (DEAD
-//                               for rows of absent contexts and for DEAD)
+//                               for rows of absent contexts and for DEAD);
+//                               then the identity column (byte d = d)
 //     Full-range quality tables (|D| ~ 31) have ~480 columns: ~23 KB against
 //     ~130 KB for a slot -> symbol table per context.
-//     Packed form, |D| <= kSmallMaxNd: MB holds plain column indices, and the
-//     columns are u64 at col_off, entry d in bits [4d, 4d + 4), so a chain
-//     step is a shift of a register instead of a shared-memory load.
+//   order-1 tiny, |D| <= kTinyMaxNd: an index d is held as its bit position
+//     5 d.
+//     [0, 4096)                 M8: u8 per slot, the slot's column
+//     [4096, + 128)             columns, u32: entry d (5 bits) at bit 5 d
+//     [4224, + 704)             the u32 table above, entry (ctx, sym) at word
+//                               30 ctx + 5 sym (the positions 5 d times 6
+//                               and 1)
 //   order-1 global (more symbols, or more columns than the image holds):
 //     [256 B] raw context -> dense index (0xFF absent), then per present
 //     context t: 4096 x u16 (sym << 8) | dense(sym), then 256 x u32
@@ -142,29 +149,28 @@ __host__ __device__ inline uint32_t dense_col_stride(int nd) { return (uint32_t)
 __host__ __device__ inline uint32_t dense_fc_bytes(int nd) {
     return (uint32_t)(((nd + 1) * (nd + 1) * 4 + 15) / 16 * 16);
 }
-__host__ __device__ inline uint32_t dense_col_off(int nd) { return kDenseM + dense_fc_bytes(nd) + 256; }
-__host__ __device__ inline bool dense_packed(int nd) { return nd <= kSmallMaxNd; }
+__host__ __device__ inline uint32_t dense_col_off(int nd) { return kDenseM + dense_fc_bytes(nd); }
 // Bytes of the table image (what is staged into shared memory).
 __host__ __device__ inline uint32_t dense_table_bytes(int nd, uint32_t ncol) {
-    return dense_packed(nd) ? dense_col_off(nd) + (8 * ncol + 15) / 16 * 16
-                            : dense_col_off(nd) + ncol * dense_col_stride(nd);
+    return dense_col_off(nd) + (ncol + 1) * dense_col_stride(nd);
 }
-// Bit-plane columns, kSmallMaxNd < |D| <= kPlaneMaxNd: after the byte
+constexpr int kTinyMaxCols = kTinyMaxNd * kTinyMaxNd + 1;
+constexpr uint32_t kTinyCol = kTotFreq;
+constexpr uint32_t kTinyFc = kTinyCol + 128;
+static_assert(4 * kTinyMaxCols <= 128, "tiny columns");
+constexpr uint32_t kTinyBytes = kTinyFc + (kTinyMaxNd * 35 + 1) * 4;
+static_assert(kTinyBytes % 16 == 0, "a table image is copied in 16-byte units");
+// Bit-plane columns, kPlaneMinNd <= |D| <= kPlaneMaxNd: after the byte
 // columns, column j's entries as five u32 planes at j * 32 (plane p, bit c =
 // bit p of the entry of context c, rotated left by p; three words of
 // padding), so that a chain step is five funnel shifts and four bit selects
 // in registers instead of a shared-memory load. The planes offset is
 // dense_table_bytes, and column j's planes sit at the byte offset of its byte
 // column (the byte stride is 32 for these |D|).
+constexpr int kPlaneMinNd = 16;
 constexpr int kPlaneMaxNd = 31;
 constexpr uint32_t kPlaneStride = 32;
-__host__ __device__ inline bool dense_planes(int nd) { return nd > kSmallMaxNd && nd <= kPlaneMaxNd; }
-// Bytes the parse needs in the arena while building the image: the packed
-// form is built from byte columns placed after it.
-__host__ __device__ inline uint32_t dense_build_bytes(int nd, uint32_t ncol) {
-    return dense_packed(nd) ? dense_table_bytes(nd, ncol) + ncol * dense_col_stride(nd)
-                            : dense_table_bytes(nd, ncol);
-}
+__host__ __device__ inline bool dense_planes(int nd) { return nd >= kPlaneMinNd && nd <= kPlaneMaxNd; }
 constexpr uint64_t kDecCtxMap = 0;
 constexpr uint64_t kDecO1Base = 256;
 constexpr uint64_t kDecO1Slot = 4096 * 2;
@@ -184,7 +190,8 @@ __host__ __device__ inline uint64_t dec_table_bytes(uint64_t src_len) {
 }
 
 // Shared-memory layout of the decode kernels.
-constexpr uint32_t kRingBytes = 2048;       // renorm-word ring, 4 x 512 B segments
+constexpr uint32_t kRingWords = 512;        // renorm-word ring
+constexpr uint32_t kRingBytes = 4 * kRingWords;  // of 32-bit elements (twice that with 64-bit ones)
 constexpr uint32_t kOutRows = 3 * kDenseMax + 1;
 
 inline uint64_t align_up(uint64_t x, uint64_t a) { return (x + a - 1) / a * a; }

@@ -1,0 +1,77 @@
+"""Order-1 decoders that guess contexts, against the oracle.
+
+The one-warp decoders walk a fixed number of columns back from each position
+and check the guessed contexts a group of eight rounds at a time
+(csrc/rans_decode.cu). These streams sit where that can go wrong: alphabets on
+both sides of the class boundaries (5 / 6 and 15 / 16 symbols with context 0),
+data whose contexts never meet (a cycle: every guess wrong, so groups are
+decoded again and the stream ends on the exact decoder), data that turns from
+one kind to the other, lengths around a round and a group, and streams and
+words at odd addresses.
+"""
+
+import numpy as np
+import pytest
+
+from fqxv_b200 import rans
+
+pytestmark = pytest.mark.gpu
+
+GROUP = 8 * 32
+LENGTHS = [1, 31, 33, GROUP - 1, GROUP + 32, 9 * GROUP + 5, 200 * GROUP + 17]
+
+
+def _symbols(rng, nsym):
+    return np.sort(rng.choice(np.arange(1, 256), nsym, replace=False)).astype(np.uint8)
+
+
+def _iid(rng, alphabet, n):
+    p = 1.0 / np.arange(1, len(alphabet) + 1)
+    return alphabet[rng.choice(len(alphabet), n, p=p / p.sum())]
+
+
+def _cycle(rng, alphabet, n):
+    """Mostly the next symbol in turn: a column permutes the contexts, so two
+    chains that start apart stay apart."""
+    step = np.where(rng.random(n) < 0.02, rng.integers(0, len(alphabet), n), 1)
+    return alphabet[np.cumsum(step) % len(alphabet)]
+
+
+def _turns(rng, alphabet, n):
+    half = n // 2
+    return np.concatenate([_iid(rng, alphabet, half), _cycle(rng, alphabet, n - half)])
+
+
+@pytest.mark.parametrize("nsym", [1, 4, 5, 13, 14, 15, 31, 40])
+@pytest.mark.parametrize("make", [_iid, _cycle, _turns])
+def test_guessed_contexts_match_oracle(orc, nsym, make):
+    import torch
+
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from fqxv_b200.batch import Codec
+
+    rng = np.random.default_rng(7 * nsym + len(make.__name__))
+    alphabet = _symbols(rng, nsym)
+    blocks = [make(rng, alphabet, n) for n in LENGTHS]
+    streams = [orc.encode(b.tobytes(), 1) for b in blocks]
+    # one filler byte in front of every second stream: odd and even addresses
+    arena, spans = b"", []
+    for i, s in enumerate(streams):
+        arena += b"\xff" * (1 + (len(arena) + i) % 2)
+        spans.append([len(arena), len(s)])
+        arena += s
+    lens = np.array([len(b) for b in blocks], dtype=np.uint64)
+    out_spans = np.stack([np.concatenate([[0], np.cumsum(lens)[:-1]]).astype(np.uint64), lens], axis=1)
+    d_src = torch.from_numpy(np.frombuffer(arena, dtype=np.uint8).copy()).to("cuda")
+    want = np.concatenate(blocks)
+    codec = Codec(0)
+    try:
+        for top_max in (0, 1000):  # with and without launch groups for the longest streams
+            codec.set_param("o1_top_max", top_max)
+            out, got, status = codec.decode_batch(d_src, spans, out_spans)
+            assert (status == 0).all() and (got == lens).all()
+            assert np.array_equal(out.cpu().numpy(), want)
+    finally:
+        codec.close()
+    assert rans.decode(streams[-1]) == blocks[-1].tobytes()
