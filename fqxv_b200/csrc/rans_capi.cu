@@ -306,10 +306,11 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
         // 32 per byte; the batch's throughput time is the sum over streams
         // of bytes x (SM cycles per byte at the class's full-GPU rate) / SMs.
         auto lat_cpb = [](const DecStream &d) {
-            return d.cls == kClsO0 ? 5.0 : d.nd <= kTinyMaxNd ? 8.0 : d.nd <= kMidMaxNd ? 11.0 : 19.5;
+            return d.cls == kClsO0 ? 4.2 : d.nd <= kTinyMaxNd ? 11.0 : d.nd <= kMidMaxNd ? 15.5 : 16.5;
         };
         auto rate_cpb = [](const DecStream &d) {
-            return d.cls == kClsO0 ? 0.9 : d.cls == kClsO1Global ? 14.0 : d.nd <= kTinyMaxNd ? 1.5 : d.nd <= kMidMaxNd ? 2.5 : 7.0;
+            return d.cls == kClsO0 ? 0.8 : d.cls == kClsO1Global ? 14.0 : d.nd <= kTinyMaxNd ? 1.8 : d.nd <= kMidMaxNd ? 3.0
+                                                                                                    : 5.0;
         };
         double bulk = 0;
         for (size_t i = 0; i < nb; i++)
@@ -341,18 +342,17 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
                                                                          : kGroupDense0 + 2;
         };
         std::vector<uint32_t> lists[kGroups];
-        uint32_t tmax[kGroups] = {}, tmaxp[kGroups] = {};
+        uint32_t tmax[kGroups] = {};
         uint64_t cbytes[kGroups] = {};
-        uint64_t maxn[kGroups] = {};
+        double maxlat[kGroups] = {};
         int ndmax[kGroups] = {};
         for (uint32_t i : ord) {
             const int g = group_of(i);
             if (g < 0) continue;
             lists[g].push_back(i);
             tmax[g] = std::max(tmax[g], ps[i].tbl_bytes);
-            tmaxp[g] = std::max(tmaxp[g], ps[i].tbl_bytes_planes);
             cbytes[g] += ps[i].src_len + ps[i].n;
-            maxn[g] = std::max<uint64_t>(maxn[g], ps[i].n);
+            maxlat[g] = std::max(maxlat[g], (double)ps[i].n * lat_cpb(ps[i]));
             ndmax[g] = std::max(ndmax[g], ps[i].nd);
         }
         int gcls[kGroups];
@@ -365,8 +365,7 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
             else if (g == kGroupMid || g == kGroupMidTop) gcls[g] = kClsO1Mid;
             else if (g == kGroupFourTop) gcls[g] = kClsO1Dense;
             else gcls[g] = (int64_t)lists[g].size() < four_max ? kClsO1Dense : kClsO1Wide;
-            // the four-warp decoder also stages the bit-plane columns
-            smem[g] = dec_smem_bytes(gcls[g], gcls[g] == kClsO1Dense ? tmaxp[g] : tmax[g], ndmax[g]);
+            smem[g] = dec_smem_bytes(gcls[g], tmax[g], ndmax[g]);
             // the groups of largest streams: one CTA per SM, alone on it
             if (is_top_group(g) && ctx->tune.o1_top_exclusive)
                 smem[g] = std::max(smem[g], dec_exclusive_smem(gcls[g], g == kGroupFourTop
@@ -374,13 +373,11 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
                                                                               : (int)ctx->tune.o1_top_small_per_sm));
         }
         // Groups are launched longest first -- by the serial time of their
-        // largest stream (rounds x cycles per round: ~620 for order-1,
-        // ~160 for order-0) -- so the streams that bound the batch take SMs
+        // largest stream (lat_cpb above) -- so the streams that bound the batch take SMs
         // before the groups that finish early.
         int glaunch[kGroups];
         for (int g = 0; g < kGroups; g++) glaunch[g] = g;
-        auto gcost = [&](int g) { return (double)maxn[g] * (g == 0 ? 160.0 : 620.0); };
-        std::stable_sort(glaunch, glaunch + kGroups, [&](int a, int b) { return gcost(a) > gcost(b); });
+        std::stable_sort(glaunch, glaunch + kGroups, [&](int a, int b) { return maxlat[a] > maxlat[b]; });
         size_t tot = 0;
         for (int g = 0; g < kGroups; g++) tot += lists[g].size();
         CK(ctx->d_order.ensure(std::max<size_t>(tot, 1) * 4, s));
@@ -431,9 +428,7 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
                     CK(cudaMemsetAsync(queue + 4 * g, 0, 4, as));
                     cudaEvent_t t0 = ctx->timer.begin(as);
                     launch_dec_run(cls, d_src, dS, dl + base[g] + j, 1, dT, d_dst, queue + 4 * g, 1,
-                                   dec_smem_bytes(cls, cls == kClsO1Dense ? ps[lists[g][j]].tbl_bytes_planes
-                                                                          : ps[lists[g][j]].tbl_bytes,
-                                                  ps[lists[g][j]].nd),
+                                   dec_smem_bytes(cls, ps[lists[g][j]].tbl_bytes, ps[lists[g][j]].nd),
                                    ctx->first_polls, mirror, as);
                     ctx->timer.end(stage, t0, as);
                 }

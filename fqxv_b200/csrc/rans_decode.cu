@@ -82,7 +82,6 @@ __global__ void __launch_bounds__(kParseThreads)
             S.nd = 0;
             S.start = 0;
             S.tbl_bytes = 0;
-            S.tbl_bytes_planes = 0;
         }
         if (status != FQXV_RANS_OK || n == 0) {
             if (tid == 0) S.status = status;
@@ -135,7 +134,6 @@ __global__ void __launch_bounds__(kParseThreads)
                 if (tid == 0) {
                     S.cls = kClsO0;
                     S.tbl_bytes = 16384;
-                    S.tbl_bytes_planes = 16384;
                 }
             }
         } else if (L < kHdr + kO1Bitmap) {
@@ -291,7 +289,7 @@ __global__ void __launch_bounds__(kParseThreads)
                         S.cls = kClsO1Dense;
                         S.nd = nd;
                         S.start = dmap[0] != 0xff ? dmap[0] : nd;
-                        S.tbl_bytes = S.tbl_bytes_planes = kTinyBytes;
+                        S.tbl_bytes = kTinyBytes;
                     }
                 } else if (dense) {
                     const uint32_t ncol = (uint32_t)s_ncol;
@@ -340,29 +338,11 @@ __global__ void __launch_bounds__(kParseThreads)
                         }
                     }
                     __syncthreads();
-                    // bit planes of every column, when they fit beside the image
-                    const bool planes = dense_planes(nd) &&
-                                        dense_table_bytes(nd, ncol) + kPlaneStride * ncol <= kDenseImageMax;
-                    if (planes) {
-                        uint32_t *PL = reinterpret_cast<uint32_t *>(T + dense_table_bytes(nd, ncol));
-                        for (uint32_t j = warp; j < ncol; j += kParseThreads / 32) {
-                            const uint32_t v = COL[j * cs + lane];
-                            uint32_t w = 0;
-#pragma unroll
-                            for (int b = 0; b < 5; b++) {
-                                const uint32_t pl = __ballot_sync(0xffffffffu, (v >> b) & 1u);
-                                if (lane == b) w = __funnelshift_l(pl, pl, b);
-                            }
-                            if (lane < 8) PL[j * (kPlaneStride / 4) + lane] = w;
-                        }
-                    }
-                    __syncthreads();
                     if (tid == 0) {
                         S.cls = kClsO1Dense;
                         S.nd = nd;
                         S.start = dmap[0] != 0xff ? dmap[0] : dead;
                         S.tbl_bytes = dense_table_bytes(nd, ncol);
-                        S.tbl_bytes_planes = S.tbl_bytes + (planes ? kPlaneStride * ncol : 0u);
                     }
                 } else {
                     if (tid < 256) T[kDecCtxMap + tid] = ctxmap[tid];
@@ -798,31 +778,6 @@ __global__ void __launch_bounds__(32, 1)
 // order-1, dense tables in shared memory (scalar.rs:180-217)
 // ---------------------------------------------------------------------------
 
-// Decode one order-1 stream whose dense tables are in shared memory, with
-// four warps (kO1Warps) per stream.
-//
-// Per round, the context chain d_i = col(slot_i)[d_{i-1}] of the 32 lanes is
-// resolved in four segments of eight: segment 0 from the known incoming
-// context, segments 1-3 for every possible incoming context at once, then
-// three dependent lookups pick the real rows. A lane turns its slot into the
-// byte offset of the slot's column once per round (one lookup in M), so each
-// chain step is one byte load from a column: the steps of all chains of a
-// segment read the same column (at most 48 bytes), not a row per context. Every warp holds its own copy
-// of the 32 states, the word position and the incoming context, and runs the
-// same renormalisation on the same words (from its own word ring), so the
-// copies never diverge and one barrier per round suffices: each thread runs
-// its share of the 3 nd speculative chains (TPL per thread, a template
-// parameter) plus, on lane 0 of every warp, segment 0; the rows go to a
-// double-buffered shared array, and after the barrier every warp resolves
-// the round itself. Only warp 0 stores the output.
-constexpr int kO1Warps = 4;
-constexpr int kO1Threads = 32 * kO1Warps;
-constexpr int kO1Workers = kO1Threads - kO1Warps;  // threads that run speculative chains
-
-__device__ __forceinline__ void named_bar(int id) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(kO1Threads) : "memory");
-}
-
 // A slot's column, as the chains of a round need it: byte columns give the
 // column's byte offset from the column base (a chain step is then one byte
 // load); tiny columns are the column itself, six 5-bit entries in a word (a
@@ -858,11 +813,10 @@ __device__ __forceinline__ void take_word(uint2 q, uint32_t srcl, uint32_t v, ui
     cb = __shfl_sync(0xffffffffu, q.y, srcl);
 }
 
-// The rounds of one order-1 dense stream (scalar.rs:202-215), shared by the
-// 4-warp and the 1-warp decoders. `D` (the decoder) gives, from every lane's
+// The rounds of one order-1 dense stream (scalar.rs:202-215) decoded by one
+// warp. `D` (the decoder) gives, from every lane's
 // column cb, this lane's context and symbol:
 //   exact(cb, ctx, d)     the right ones
-//   D::kGuess             whether guess() exists; else every round is exact()
 //   guess<P>(cb, ctx, d)  likely ones (P: the round's parity); returns whether
 //                         this lane's context is its neighbour's symbol (a
 //                         round is right when that holds in every lane)
@@ -871,7 +825,6 @@ __device__ __forceinline__ void take_word(uint2 q, uint32_t srcl, uint32_t v, ui
 //   entry(ctx, d)         ((freq - 1) << 20) | (cum << 8) | byte, kDeadEntry
 //                         for what a context without a table "decodes"
 //   next(d)               takes the round's last symbol as the next context
-// `store` says whether this warp writes the output.
 //
 // Rounds that cannot run out of words (and are not the first or the partial
 // last round) take the fast path, kO1Group rounds per ring advance; a context
@@ -894,7 +847,7 @@ static_assert(32 * kO1Group + 64 <= 3 * kSegWords, "a group's words are resident
 
 template <class Col, class D>
 __device__ __forceinline__ int o1_rounds(DecStream &S, WordRing<Col> &R, uint8_t *__restrict__ out, uint32_t lt,
-                                         bool store, uint32_t x, D &dec) {
+                                         uint32_t x, D &dec) {
     const Col &C = R.make;
     const int lane = threadIdx.x & 31;
     const uint64_t n = S.n;
@@ -932,7 +885,7 @@ __device__ __forceinline__ int o1_rounds(DecStream &S, WordRing<Col> &R, uint8_t
                 break;
             }
             if (active) {
-                if (store) out[i] = (uint8_t)e;
+                out[i] = (uint8_t)e;
                 x = v;
             }
             r++;
@@ -955,7 +908,7 @@ __device__ __forceinline__ int o1_rounds(DecStream &S, WordRing<Col> &R, uint8_t
             const uint32_t mask = __ballot_sync(0xffffffffu, need);
             uint32_t xw, cbw;
             take_word(q, __popc(mask & lt), v, xw, cbw);
-            if (store) *o = (uint8_t)e;
+            *o = (uint8_t)e;
             top = max(top, e);
             x = need ? xw : v;
             cb = need ? cbw : cbv;
@@ -972,8 +925,7 @@ __device__ __forceinline__ int o1_rounds(DecStream &S, WordRing<Col> &R, uint8_t
         for (int64_t c = 0; c < cnt; c += kO1Group) {
             R.advance(wp);
             const int m = (int)(cnt - c < kO1Group ? cnt - c : kO1Group);
-            if constexpr (D::kGuess) {
-                if (m == kO1Group && dec.guessing()) {
+            if (m == kO1Group && dec.guessing()) {
                     const uint32_t x0 = x, cb0 = cb, top0 = top;
                     const D before = dec;
                     bool wrong = false;
@@ -994,9 +946,6 @@ __device__ __forceinline__ int o1_rounds(DecStream &S, WordRing<Col> &R, uint8_t
                         exact_rounds(m);
                     }
                     dec.guessed(right);
-                } else {
-                    exact_rounds(m);
-                }
             } else {
                 exact_rounds(m);
             }
@@ -1008,27 +957,6 @@ __device__ __forceinline__ int o1_rounds(DecStream &S, WordRing<Col> &R, uint8_t
     }
     return status;
 }
-
-// An exact-only decoder from a function (cb, ctx, d) and its entry table.
-template <class Exact>
-struct ExactDecoder {
-    static constexpr bool kGuess = false;
-    const uint32_t *FC;
-    uint32_t stride;
-    Exact exact;
-    __device__ __forceinline__ uint32_t entry(uint32_t ctx, uint32_t d) const { return FC[ctx * stride + d]; }
-    __device__ __forceinline__ void next(uint32_t) {}
-};
-
-// Rows of the speculative chains, 16 bytes each: the eight chain values
-// (d_0 the top byte of .x, d_7 the low byte of .y) and, in .z, the byte
-// offset of the row the next segment continues from (the DEAD row when the
-// chain ends in a context without a table), so that resolving a round is
-// three dependent loads and no index arithmetic. Row kDeadRow repeats DEAD;
-// row kPadRow takes the stores of threads without a task.
-constexpr uint32_t kDeadRow = 3 * kDenseMax;
-constexpr uint32_t kPadRow = kDeadRow + 1;
-static_assert(kPadRow <= kOutRows, "row array too small");
 
 // The parts of a dense table image in shared memory.
 struct DenseImage {
@@ -1047,194 +975,275 @@ struct DenseImage {
           dead((uint32_t)nd) {}
 };
 
-template <int TPL>
-__device__ __forceinline__ int o1d_stream(DecStream &S, const uint8_t *__restrict__ sm, WordRing<ByteCols> &R,
-                                          uint4 (*__restrict__ rows)[kOutRows + 1], uint8_t *__restrict__ out,
-                                          uint32_t lt) {
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int nd = S.nd;
-    const DenseImage I(sm, nd);
-    const uint32_t dead = I.dead;
-    const int nspec = 3 * nd;
-    // This thread's chains: lane 0 of each warp runs segment 0 (q = 0); the
-    // other threads split the speculative tasks u = (seg - 1) nd + c.
-    const int worker = warp * 31 + lane - 1;
-    uint32_t seg_q[TPL], c_q[TPL], idx_q[TPL], nbase_q[TPL];
-#pragma unroll
-    for (int q = 0; q < TPL; q++) {
-        const int u = worker + kO1Workers * q;
-        const bool valid = lane != 0 && u < nspec;
-        seg_q[q] = lane == 0 ? 0u : valid ? (uint32_t)(1 + u / nd) : 1u;
-        c_q[q] = valid ? (uint32_t)(u % nd) : 0u;
-        idx_q[q] = valid ? (uint32_t)u : kPadRow;
-        nbase_q[q] = seg_q[q] * (uint32_t)nd;  // first row of the next segment
-    }
-    const uint8_t *COL = I.COL;
-    const uint32_t deadw = 0x01010101u * dead;
-    if (tid == 0) {
-        rows[0][kDeadRow] = make_uint4(deadw, deadw, kDeadRow * 16u, 0u);
-        rows[1][kDeadRow] = make_uint4(deadw, deadw, kDeadRow * 16u, 0u);
-    }
-    const uint32_t x = S.states[lane];
-    uint32_t din = (uint32_t)S.start;
-    const int seg = lane >> 3, pos = lane & 7;
-    const uint32_t shd = 24u - 8u * (uint32_t)(pos & 3);        // byte pos of a row half
-    const uint32_t shc = 24u - 8u * (uint32_t)((pos + 3) & 3);  // byte pos - 1
-    uint32_t buf = 0;
+// ---------------------------------------------------------------------------
+// order-1, four warps per stream (wide alphabets whose serial time bounds a
+// batch)
+// ---------------------------------------------------------------------------
 
-    // One round: the chains of this thread, the barrier, then the resolved
-    // symbol d and context ctx of this lane.
-    auto exact = [&](uint32_t cb, uint32_t &ctx, uint32_t &d) {
-        uint4 mine[TPL];
+// Only the context runs serially through a stream's positions (and, behind
+// it, the count of words taken): the rest of a state's step has 32 positions
+// of slack. So warp w owns states 8 w .. 8 w + 7 (lane l computes state
+// l & 7, four times over), and the warps run a quarter round apart, handing
+// on two numbers, each through a slot in shared memory and a named barrier
+// (arrive by the giver, sync by the taker): the last symbol, then the word
+// position.
+//
+// While its context is on the way a warp turns its eight columns into
+// functions of it: lane c holds what context c becomes. f_k is one byte of
+// column k per lane; the functions of the first k columns are compositions,
+// and composing is a shuffle (h[c] = g[f[c]]), three levels for eight columns.
+// When the context arrives, three shuffles give all eight symbols, and the
+// context goes on to the next warp at once. With contexts of 32 and up (HI,
+// |D| > 32) a function takes two registers and a composition four shuffles;
+// there each lane walks columns 0-3 and 4-7 from contexts lane and lane + 32
+// by byte loads, and only the second walk is composed after the first.
+//
+// What bounds it is a warp's own loop, about 130 instructions, most of them
+// in one dependent chain (a hop to the next warp is ~85 cycles, four a round
+// ~340). One stream, cycles per round: full-range quality (|D| = 31) 529, ONT
+// quality (39) 601, random walk (41) 598. Before, every warp held all 32
+// states, ran a segment's chains from every context and followed three rows
+// of shared memory behind a barrier: 642, 614 and 615.
+constexpr int kO1Warps = 4;
+constexpr int kO1Threads = 32 * kO1Warps;
+
+// prmt with its full selectors (__byte_perm keeps three bits of each): 8 gives
+// the sign of byte 0, so values below 128 come zero-extended.
+__device__ __forceinline__ uint32_t pick_byte(uint32_t lo, uint32_t hi, uint32_t sel) {
+    uint32_t r;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(lo), "r"(hi), "r"(sel));
+    return r;
+}
+__device__ __forceinline__ void bar_arrive(int id) { asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory"); }
+__device__ __forceinline__ void bar_take(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+
+struct RelayShared {
+    uint32_t x[kStates];          // states between runs of fast rounds
+    volatile uint32_t ctx[4];     // slot w: handed on by warp w
+    volatile uint32_t pos[4];
+    uint64_t wp, r;
+    int64_t cnt;                  // fast rounds of the next run; 0: done
+    uint32_t din;
+    uint32_t dead;                // a context without a table was met
+};
+
+// cnt fast rounds of warp w; x0: its state of the first, din / wp: the first
+// round's context and word position. The caller has made sure that the words
+// of cnt rounds are there. Returns the word position after the run and leaves
+// the last symbol in din (warp 0 only), the state in x.
+template <bool HI>
+__device__ __forceinline__ void relay_rounds(RelayShared &sh, const DenseImage &I, WordRing<ByteCols> &R, int w,
+                                             uint32_t &x, uint32_t &din, uint64_t &wp, int64_t cnt,
+                                             uint8_t *__restrict__ op, uint32_t &top) {
+    const int lane = threadIdx.x & 31, k = lane & 7;
+    const ByteCols &C = R.make;
+    const int from = (w + 3) & 3;
+    const uint32_t below = (1u << k) - 1u;
+    const uint32_t pick_d = 0x8880u | (uint32_t)k;                       // byte k, zero-extended
+    const uint32_t pick_c = 0x8880u | (uint32_t)(k > 0 ? k - 1 : 0);     // byte k - 1
+    const uint32_t c0 = min((uint32_t)lane, I.dead), c1 = HI ? min((uint32_t)lane + 32u, I.dead) : 0u;
+    uint32_t cb = C.look(x & (kTotFreq - 1));
+    uint32_t pos = (uint32_t)wp;
+    op += 8 * w + k;
+    for (int64_t i = 0; i < cnt; i += 8) {
+        wp += (uint32_t)(pos - (uint32_t)wp);
+        R.advance(wp);
+        const int m = (int)(cnt - i < 8 ? cnt - i : 8);
+        for (int g = 0; g < m; g++) {
+            const bool first = w == 0 && i + g == 0;
+            uint32_t in = din, last, a, b, o[8];
 #pragma unroll
-        for (int q = 0; q < TPL; q++) {
-            uint32_t sl[8];
+            for (int q = 0; q < 8; q++) o[q] = __shfl_sync(0xffffffffu, cb, q);
+            auto take_ctx = [&] {
+                if (first) return;
+                bar_take(1 + from);
+                in = sh.ctx[from];
+            };
+            if constexpr (!HI) {
+                uint32_t f[8];
 #pragma unroll
-            for (int k = 0; k < 8; k++) sl[k] = __shfl_sync(0xffffffffu, cb, 8 * seg_q[q] + k);
-            uint32_t dd = (q == 0 && lane == 0) ? din : c_q[q];
-            uint32_t hi = 0, lo = 0;
+                for (int q = 0; q < 8; q++) f[q] = I.COL[o[q] + c0];
+                const uint32_t p1 = __shfl_sync(0xffffffffu, f[1], f[0]);
+                const uint32_t q3 = __shfl_sync(0xffffffffu, f[3], f[2]);
+                const uint32_t q5 = __shfl_sync(0xffffffffu, f[5], f[4]);
+                const uint32_t q7 = __shfl_sync(0xffffffffu, f[7], f[6]);
+                const uint32_t p3 = __shfl_sync(0xffffffffu, q3, p1);
+                const uint32_t r7 = __shfl_sync(0xffffffffu, q7, q5);
+                const uint32_t p2 = __shfl_sync(0xffffffffu, f[2], p1);
+                const uint32_t r6 = __shfl_sync(0xffffffffu, f[6], q5);
+                const uint32_t p7 = __shfl_sync(0xffffffffu, r7, p3);
+                const uint32_t p4 = __shfl_sync(0xffffffffu, f[4], p3);
+                const uint32_t p5 = __shfl_sync(0xffffffffu, q5, p3);
+                const uint32_t p6 = __shfl_sync(0xffffffffu, r6, p3);
+                a = (f[0] + 256u * p1) + 65536u * (p2 + 256u * p3);
+                b = (p4 + 256u * p5) + 65536u * (p6 + 256u * p7);
+                // all of the above before the wait
+                asm volatile("" ::"r"(a), "r"(b), "r"(p7));
+                take_ctx();
+                last = __shfl_sync(0xffffffffu, p7, in);
+                a = __shfl_sync(0xffffffffu, a, in);
+                b = __shfl_sync(0xffffffffu, b, in);
+            } else {
+                // positions 0-3 and 4-7 as chains of their own, side by side,
+                // then the second after the first
+                uint32_t t0 = c0, t1 = c1, u0 = c0, u1 = c1, a0 = 0, a1 = 0, b0 = 0, b1 = 0;
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                dd = COL[sl[k] + dd];
-                hi = hi * 256u + dd;
+                for (int q = 0; q < 4; q++) {
+                    t0 = I.COL[o[q] + t0];
+                    t1 = I.COL[o[q] + t1];
+                    u0 = I.COL[o[q + 4] + u0];
+                    u1 = I.COL[o[q + 4] + u1];
+                    a0 += t0 << (8 * q);
+                    a1 += t1 << (8 * q);
+                    b0 += u0 << (8 * q);
+                    b1 += u1 << (8 * q);
+                }
+                // what a function held as (lo: contexts 0-31, hi: 32 and up)
+                // makes of context c
+                auto value = [](uint32_t lo, uint32_t hi, uint32_t c) {
+                    const uint32_t l = __shfl_sync(0xffffffffu, lo, c), h = __shfl_sync(0xffffffffu, hi, c);
+                    return c < 32u ? l : h;
+                };
+                const uint32_t p0 = value(b0, b1, t0), p1 = value(b0, b1, t1);
+                asm volatile("" ::"r"(a0), "r"(a1), "r"(p0), "r"(p1));
+                take_ctx();
+                b = value(p0, p1, in);
+                last = b >> 24;
+                a = value(a0, a1, in);
             }
-#pragma unroll
-            for (int k = 4; k < 8; k++) {
-                dd = COL[sl[k] + dd];
-                lo = lo * 256u + dd;
+            if (lane == 0) sh.ctx[w] = last;
+            __syncwarp();
+            bar_arrive(1 + w);
+            const uint32_t d = pick_byte(a, b, pick_d);
+            const uint32_t prev = pick_byte(a, b, pick_c);
+            const uint32_t ctx = k == 0 ? in : prev;
+            const uint32_t e = I.FC[ctx * I.stride + d];
+            // taken while the entry is on its way
+            if (!first) {
+                bar_take(5 + from);
+                pos = sh.pos[from];
             }
-            mine[q] = make_uint4(hi, lo, 16u * (dd == dead ? kDeadRow : nbase_q[q] + dd), 0u);
+            const uint32_t ahead = R.at(pos + k);
+            const uint32_t xs = x >> kScaleBits;
+            const uint32_t v = (e >> 20) * xs + (xs + (x & (kTotFreq - 1)) - ((e >> 8) & (kTotFreq - 1)));
+            const uint32_t cbv = C.look(v & (kTotFreq - 1));
+            const bool need = v < kRansL;
+            const uint32_t mask = __ballot_sync(0xffffffffu, need) & 0xffu;
+            pos += __popc(mask);
+            if (lane == 0) sh.pos[w] = pos;
+            __syncwarp();
+            bar_arrive(5 + w);
+            const uint32_t q = __shfl_sync(0xffffffffu, ahead, __popc(mask & below));
+            if (lane < 8) *op = (uint8_t)e;
+            op += 32;
+            top = max(top, e);
+            x = need ? __byte_perm(q, v, 0x5410) : v;
+            cb = need ? (q >> 12) & ~15u : cbv;
         }
-        uint4 *rb = rows[buf];
-#pragma unroll
-        for (int q = 0; q < TPL; q++)
-            if (q > 0 || lane != 0) rb[idx_q[q]] = mine[q];
-        uint4 r0;
-        r0.x = __shfl_sync(0xffffffffu, mine[0].x, 0);
-        r0.y = __shfl_sync(0xffffffffu, mine[0].y, 0);
-        r0.z = __shfl_sync(0xffffffffu, mine[0].z, 0);
-        named_bar(1);
-        const uint8_t *rbb = reinterpret_cast<const uint8_t *>(rb);
-        const uint4 r1 = *reinterpret_cast<const uint4 *>(rbb + r0.z);
-        const uint4 r2 = *reinterpret_cast<const uint4 *>(rbb + r1.z);
-        const uint32_t rx = seg == 0 ? r0.x : seg == 1 ? r1.x : r2.x;
-        const uint32_t ry = seg == 0 ? r0.y : seg == 1 ? r1.y : r2.y;
-        const uint32_t ine = seg == 0 ? din : seg == 1 ? (r0.y & 0xffu) : (r1.y & 0xffu);
-        const uint4 r3 = *reinterpret_cast<const uint4 *>(rbb + r2.z);
-        const uint32_t row_x = seg == 3 ? r3.x : rx;
-        const uint32_t row_y = seg == 3 ? r3.y : ry;
-        const uint32_t in = seg == 3 ? (r2.y & 0xffu) : ine;
-        d = ((pos < 4 ? row_x : row_y) >> shd) & 0xffu;
-        ctx = pos == 0 ? in : ((pos <= 4 ? row_x : row_y) >> shc) & 0xffu;
-        din = r3.y & 0xffu;
-        buf ^= 1u;
-    };
-
-    ExactDecoder<decltype(exact)> dec{I.FC, I.stride, exact};
-    return o1_rounds(S, R, out, lt, warp == 0, x, dec);
+    }
+    if (w == 0) {
+        // takes what warp 3 handed on in the last round
+        bar_take(1 + from);
+        din = sh.ctx[from];
+        bar_take(5 + from);
+        pos = sh.pos[from];
+    }
+    wp += (uint32_t)(pos - (uint32_t)wp);
 }
 
-// Four-warp decode of a stream with bit-plane columns (kPlaneMinNd <= |D| <=
-// kPlaneMaxNd). Warp w >= 1 runs segment w for every incoming context, lane
-// c from context c, and lane 31 of every warp runs segment 0 from the known
-// context, so each warp has the first segment's row in registers. A chain
-// step looks its next context up in the column's five bit planes (loaded
-// into registers once per round): plane p rotated right by the context puts
-// the entry's bit p at bit p, and four bit selects merge the five. Rows are
-// (segment, context) pairs, 32 per segment; row (s, 31) is the DEAD row
-// when |D| = 31 (the DEAD context is then 31, whose lane runs segment 0)
-// and is never reached otherwise. The round is then resolved as in
-// o1d_stream: three dependent row loads after the barrier.
-__device__ __forceinline__ int o1p_stream(DecStream &S, const uint8_t *__restrict__ sm, WordRing<ByteCols> &R,
-                                          uint4 (*__restrict__ rows)[kOutRows + 1], uint8_t *__restrict__ out,
-                                          uint32_t lt) {
-    static_assert(4 * 32 <= kOutRows + 1, "row array holds four segments of 32 rows");
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int nd = S.nd;
-    const DenseImage I(sm, nd);
-    const uint32_t dead = I.dead;
-    const uint8_t *PL = sm + S.tbl_bytes;
-    const uint32_t myseg = lane == 31 ? 0u : (uint32_t)warp;
-    const bool writer = warp >= 1 && lane < 31;
-    const uint32_t nbase = 32u * (myseg + 1u);  // row of context 0 in the next segment
-    const uint32_t deadw = 0x01010101u * dead;
-    if (tid < 6) {
-        const uint32_t sg = 1u + (uint32_t)(tid % 3);
-        rows[tid / 3][32u * sg + 31u] = make_uint4(deadw, deadw, 16u * (32u * (sg + 1u) + 31u), 0u);
+// One stream: warp 0 alone decodes the rounds that need every check of
+// scalar.rs:202-215 (the first, the partial last one and those whose words
+// might run out), one position after another; the runs of rounds between
+// them go through the relay.
+template <bool HI>
+__device__ __forceinline__ int relay_stream(RelayShared &sh, DecStream &S, const DenseImage &I,
+                                            WordRing<ByteCols> &R, uint8_t *__restrict__ out, uint32_t lt) {
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    const uint64_t n = S.n, navail = S.words_len / 2;
+    const uint64_t rounds = (n + 31) / 32, full = n / 32;
+    uint64_t wp = 0, r = 0;
+    uint32_t din = (uint32_t)S.start, top = 0, x = S.states[lane];
+    int status = FQXV_RANS_OK;
+    for (;;) {
+        if (w == 0) {
+            int64_t cnt = 0;
+            while (r < rounds && status == FQXV_RANS_OK) {
+                const int64_t spare = (int64_t)navail - (int64_t)wp - 64;
+                cnt = spare > 0 ? spare / 32 : 0;
+                const int64_t left_full = r < full ? (int64_t)(full - r) : 0;
+                if (cnt > left_full) cnt = left_full;
+                if (r != 0 && cnt > 0) break;
+                cnt = 0;
+                R.advance(wp);
+                const uint64_t i = r * 32 + lane;
+                const bool active = i < n;
+                const uint32_t slot = x & (kTotFreq - 1);
+                const uint32_t cb = R.make.look(slot);
+                uint32_t t = din, ctx = 0, d = 0;
+                for (int k = 0; k < 32; k++) {
+                    if (lane == k) ctx = t;
+                    t = I.COL[__shfl_sync(0xffffffffu, cb, k) + t];
+                    if (lane == k) d = t;
+                }
+                din = t;
+                const uint32_t e = I.FC[ctx * I.stride + d];
+                const uint32_t deadmask = __ballot_sync(0xffffffffu, active && e == kDeadEntry);
+                const int absent_at = deadmask ? __ffs(deadmask) - 1 : 32;
+                const bool valid = active && lane < absent_at;
+                uint32_t v = ((e >> 20) + 1) * (x >> kScaleBits) + slot - ((e >> 8) & (kTotFreq - 1));
+                const bool need = valid && v < kRansL;
+                if (!renorm_round(v, need, R, wp, navail, lt, r == 0)) {
+                    status = FQXV_RANS_E_TRUNCATED;
+                    break;
+                }
+                if (absent_at < 32) {
+                    status = FQXV_RANS_E_ABSENT_CONTEXT;
+                    break;
+                }
+                if (active) {
+                    out[i] = (uint8_t)e;
+                    x = v;
+                }
+                r++;
+            }
+            sh.x[lane] = x;
+            if (lane == 0) {
+                sh.wp = wp;
+                sh.r = r;
+                sh.din = din;
+                sh.cnt = cnt;
+                sh.dead = 0;
+            }
+        }
+        __syncthreads();
+        const int64_t cnt = sh.cnt;
+        if (cnt == 0) return status;  // of warp 0
+        wp = sh.wp;
+        r = sh.r;
+        din = sh.din;
+        x = sh.x[8 * w + (lane & 7)];
+        __syncthreads();  // sh.x is read before it is written again
+        relay_rounds<HI>(sh, I, R, w, x, din, wp, cnt, out + r * 32, top);
+        if (lane < 8) sh.x[8 * w + lane] = x;
+        if (__any_sync(0xffffffffu, top == kDeadEntry) && lane == 0) sh.dead = 1;
+        __syncthreads();
+        r += (uint64_t)cnt;
+        if (w == 0) {
+            x = sh.x[lane];
+            if (sh.dead) status = FQXV_RANS_E_ABSENT_CONTEXT;
+        }
     }
-    uint32_t din = (uint32_t)S.start;
-    const int seg = lane >> 3, pos = lane & 7;
-    const uint32_t shd = 24u - 8u * (uint32_t)(pos & 3);
-    const uint32_t shc = 24u - 8u * (uint32_t)((pos + 3) & 3);
-    uint32_t buf = 0;
-
-    auto exact = [&](uint32_t cb, uint32_t &ctx, uint32_t &d) {
-        uint32_t q[8][5];
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const uint32_t off = __shfl_sync(0xffffffffu, cb, 8 * myseg + k);
-            const uint4 a = *reinterpret_cast<const uint4 *>(PL + off);
-            q[k][0] = a.x;
-            q[k][1] = a.y;
-            q[k][2] = a.z;
-            q[k][3] = a.w;
-            q[k][4] = *reinterpret_cast<const uint32_t *>(PL + off + 16);
-        }
-        uint32_t dd = lane == 31 ? din : (uint32_t)lane;
-        uint32_t hi = 0, lo = 0;
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const uint32_t t0 = __funnelshift_r(q[k][0], q[k][0], dd);
-            const uint32_t t1 = __funnelshift_r(q[k][1], q[k][1], dd);
-            const uint32_t t2 = __funnelshift_r(q[k][2], q[k][2], dd);
-            const uint32_t t3 = __funnelshift_r(q[k][3], q[k][3], dd);
-            const uint32_t t4 = __funnelshift_r(q[k][4], q[k][4], dd);
-            const uint32_t a = (t0 & 1u) | (t1 & ~1u);
-            const uint32_t b = (t2 & 7u) | (t3 & ~7u);
-            const uint32_t c = (a & 3u) | (b & ~3u);
-            // bits above 4 are left over from the planes: a funnel shift
-            // uses its amount mod 32, and the row keeps the clean value
-            dd = (c & 15u) | (t4 & ~15u);
-            if (k < 4) hi = (hi << 8) | (dd & 31u);
-            else lo = (lo << 8) | (dd & 31u);
-        }
-        const uint32_t nx = 16u * (nbase + (dd & 31u));
-        uint4 *rb = rows[buf];
-        if (writer) rb[32 * warp + lane] = make_uint4(hi, lo, nx, 0u);
-        uint4 r0;
-        r0.x = __shfl_sync(0xffffffffu, hi, 31);
-        r0.y = __shfl_sync(0xffffffffu, lo, 31);
-        r0.z = __shfl_sync(0xffffffffu, nx, 31);
-        named_bar(1);
-        const uint8_t *rbb = reinterpret_cast<const uint8_t *>(rb);
-        const uint4 r1 = *reinterpret_cast<const uint4 *>(rbb + r0.z);
-        const uint4 r2 = *reinterpret_cast<const uint4 *>(rbb + r1.z);
-        const uint32_t rx = seg == 0 ? r0.x : seg == 1 ? r1.x : r2.x;
-        const uint32_t ry = seg == 0 ? r0.y : seg == 1 ? r1.y : r2.y;
-        const uint32_t ine = seg == 0 ? din : seg == 1 ? (r0.y & 0xffu) : (r1.y & 0xffu);
-        const uint4 r3 = *reinterpret_cast<const uint4 *>(rbb + r2.z);
-        const uint32_t row_x = seg == 3 ? r3.x : rx;
-        const uint32_t row_y = seg == 3 ? r3.y : ry;
-        const uint32_t in = seg == 3 ? (r2.y & 0xffu) : ine;
-        d = ((pos < 4 ? row_x : row_y) >> shd) & 0xffu;
-        ctx = pos == 0 ? in : ((pos <= 4 ? row_x : row_y) >> shc) & 0xffu;
-        din = r3.y & 0xffu;
-        buf ^= 1u;
-    };
-
-    ExactDecoder<decltype(exact)> dec{I.FC, I.stride, exact};
-    return o1_rounds(S, R, out, lt, warp == 0, S.states[lane], dec);
 }
 
-__global__ void __launch_bounds__(kO1Threads, 1)
+__global__ void __launch_bounds__(kO1Threads, 4)
     dec_o1d_kernel(const uint8_t *__restrict__ src, DecStream *__restrict__ streams,
                    const uint32_t *__restrict__ list, int nlist, const uint8_t *__restrict__ tbl,
                    uint8_t *__restrict__ dst, int *__restrict__ queue, uint32_t ring_off,
                    uint32_t first_polls, uint8_t *__restrict__ mirror) {
     extern __shared__ __align__(128) uint8_t sm[];
     __shared__ __align__(8) uint64_t bar;
-    __shared__ __align__(16) uint4 s_rows[2][kOutRows + 1];
-    __shared__ int s_job, s_ok, s_stuck;
+    __shared__ RelayShared sh;
+    __shared__ int s_job, s_ok, s_stuck, s_status;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t lt = lanemask_lt();
     TableStager st;
@@ -1251,7 +1260,7 @@ __global__ void __launch_bounds__(kO1Threads, 1)
         if (warp == 0) {
             bool ok = false;
             if (!s_stuck) {
-                st.issue(sm, tbl + S.tbl_off, S.tbl_bytes_planes);
+                st.issue(sm, tbl + S.tbl_off, S.tbl_bytes);
                 ok = st.wait(first_polls);
                 if (!ok && !st.drain() && lane == 0) s_stuck = 1;
             }
@@ -1265,13 +1274,14 @@ __global__ void __launch_bounds__(kO1Threads, 1)
         WordRing<ByteCols> R(ByteCols{I.M8, I.MB, dense_col_stride(S.nd)});
         R.init(src + S.words_off, S.words_len, sm + ring_off + warp * kRingBytes);
         uint8_t *out = dst + S.dst_off;
-        const int tpl = (3 * S.nd + kO1Workers - 1) / kO1Workers;
-        const int status = S.tbl_bytes_planes > S.tbl_bytes ? o1p_stream(S, sm, R, s_rows, out, lt)
-                           : tpl <= 1                       ? o1d_stream<1>(S, sm, R, s_rows, out, lt)
-                                                            : o1d_stream<2>(S, sm, R, s_rows, out, lt);
-        if (tid == 0) S.status = status;
+        // 32 symbols leave no lane for DEAD, and need none: a stream that meets
+        // it has failed, and any context may follow.
+        const int status = S.nd <= 32 ? relay_stream<false>(sh, S, I, R, out, lt)
+                                      : relay_stream<true>(sh, S, I, R, out, lt);
+        if (tid == 0) s_status = S.status = status;
         __syncthreads();
-        if (mirror && status == FQXV_RANS_OK) mirror_out(out, mirror + S.dst_off, S.n, tid, kO1Threads);
+        if (mirror && s_status == FQXV_RANS_OK) mirror_out(out, mirror + S.dst_off, S.n, tid, kO1Threads);
+        __syncthreads();
     }
 }
 
@@ -1314,7 +1324,6 @@ struct GuessTrust {
 __device__ __forceinline__ uint32_t tiny_step(uint32_t col, uint32_t at) { return __funnelshift_r(col, col, at); }
 
 struct TinyDecoder : GuessTrust {
-    static constexpr bool kGuess = true;
     static constexpr int kBack = 16;
     // Exchange array: two buffers (by the round's parity) of two copies, the
     // second one word later, so that a lane's columns are aligned pairs in
@@ -1483,7 +1492,6 @@ struct RowDecoder {
 // 0.86 of full-range quality's, whose streams then go to exact() for good.
 template <int TPL>
 struct WideDecoder : RowDecoder<TPL>, GuessTrust {
-    static constexpr bool kGuess = true;
     static constexpr int kBack = 10;
     static constexpr int kBuf = kBack + 32;
     static constexpr uint32_t kBytes = 2 * kBuf * 4;
@@ -1518,7 +1526,6 @@ struct WideDecoder : RowDecoder<TPL>, GuessTrust {
 // at, zero here, so each half gives the entry or zero and the two are or-ed
 // (bits above the low four of a selector do no harm: only byte 0 counts).
 struct MidDecoder : RowDecoder<2>, GuessTrust {
-    static constexpr bool kGuess = true;
     static constexpr int kBack = 16;
     // Exchange array: kBack identity columns, then the lanes' (two buffers).
     static constexpr int kBuf = kBack + 32;
@@ -1560,7 +1567,7 @@ template <int TPL>
 __device__ __forceinline__ int o1w_stream(DecStream &S, const uint8_t *__restrict__ sm, WordRing<ByteCols> &R,
                                           uint4 *rows, uint8_t *xch, uint8_t *__restrict__ out, uint32_t lt) {
     WideDecoder<TPL> dec(S, sm, rows, reinterpret_cast<uint32_t *>(xch));
-    return o1_rounds(S, R, out, lt, true, S.states[threadIdx.x & 31], dec);
+    return o1_rounds(S, R, out, lt, S.states[threadIdx.x & 31], dec);
 }
 
 // The one-warp order-1 decoders: tiny alphabets, up to kMidMaxNd symbols, and
@@ -1609,7 +1616,7 @@ __global__ void __launch_bounds__(32, kCls == kClsO1Wide ? 8 : 16)
                 WordWith<TinyCols>(TinyCols{sm, reinterpret_cast<const uint32_t *>(sm + kTinyCol)}));
             R.init(src + S.words_off, S.words_len, sm + ring_off);
             TinyDecoder dec(S, sm, reinterpret_cast<uint32_t *>(s_xch));
-            status = o1_rounds(S, R, out, lt, true, S.states[lane], dec);
+            status = o1_rounds(S, R, out, lt, S.states[lane], dec);
         } else {
             const DenseImage I(sm, S.nd);
             WordRing<ByteCols> R(ByteCols{I.M8, I.MB, dense_col_stride(S.nd)});
@@ -1617,7 +1624,7 @@ __global__ void __launch_bounds__(32, kCls == kClsO1Wide ? 8 : 16)
             uint4 *rows = reinterpret_cast<uint4 *>(sm + ring_off - wide_rows_bytes(S.nd));
             if constexpr (kCls == kClsO1Mid) {
                 MidDecoder dec(S, sm, rows, reinterpret_cast<uint4 *>(s_xch));
-                status = o1_rounds(S, R, out, lt, true, S.states[lane], dec);
+                status = o1_rounds(S, R, out, lt, S.states[lane], dec);
             } else {
                 const int tpl = (S.nd + kWideLanes - 1) / kWideLanes;
                 status = tpl <= 2   ? o1w_stream<2>(S, sm, R, rows, s_xch, out, lt)

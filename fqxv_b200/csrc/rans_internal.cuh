@@ -88,8 +88,6 @@ struct DecStream {
     int32_t nd;                  // dense format: |D| (symbols and contexts), DEAD = nd
     int32_t start;               // dense format: index of context 0 (DEAD when absent)
     uint32_t tbl_bytes;          // bytes of the table image staged into shared memory
-    uint32_t tbl_bytes_planes;   // dense format with bit-plane columns: image + planes
-                                 // (the four-warp decoder stages these); else tbl_bytes
     uint32_t states[kStates];
 };
 
@@ -160,17 +158,6 @@ constexpr uint32_t kTinyFc = kTinyCol + 128;
 static_assert(4 * kTinyMaxCols <= 128, "tiny columns");
 constexpr uint32_t kTinyBytes = kTinyFc + (kTinyMaxNd * 35 + 1) * 4;
 static_assert(kTinyBytes % 16 == 0, "a table image is copied in 16-byte units");
-// Bit-plane columns, kPlaneMinNd <= |D| <= kPlaneMaxNd: after the byte
-// columns, column j's entries as five u32 planes at j * 32 (plane p, bit c =
-// bit p of the entry of context c, rotated left by p; three words of
-// padding), so that a chain step is five funnel shifts and four bit selects
-// in registers instead of a shared-memory load. The planes offset is
-// dense_table_bytes, and column j's planes sit at the byte offset of its byte
-// column (the byte stride is 32 for these |D|).
-constexpr int kPlaneMinNd = 16;
-constexpr int kPlaneMaxNd = 31;
-constexpr uint32_t kPlaneStride = 32;
-__host__ __device__ inline bool dense_planes(int nd) { return nd >= kPlaneMinNd && nd <= kPlaneMaxNd; }
 constexpr uint64_t kDecCtxMap = 0;
 constexpr uint64_t kDecO1Base = 256;
 constexpr uint64_t kDecO1Slot = 4096 * 2;
@@ -192,7 +179,6 @@ __host__ __device__ inline uint64_t dec_table_bytes(uint64_t src_len) {
 // Shared-memory layout of the decode kernels.
 constexpr uint32_t kRingWords = 512;        // renorm-word ring
 constexpr uint32_t kRingBytes = 4 * kRingWords;  // of 32-bit elements (twice that with 64-bit ones)
-constexpr uint32_t kOutRows = 3 * kDenseMax + 1;
 
 inline uint64_t align_up(uint64_t x, uint64_t a) { return (x + a - 1) / a * a; }
 
