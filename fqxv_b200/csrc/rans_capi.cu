@@ -156,7 +156,9 @@ int encode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
         nmax = std::max<uint64_t>(nmax, hb[i].n);
     }
     const bool tail = (double)nmax > 4.0 * (double)nsum / (double)nb;
-    const int run_grid = ctx->sms * (int)(tail ? ctx->tune.enc_run_ctas_per_sm : ctx->tune.enc_run_ctas_per_sm_uniform);
+    // (the parameters count jobs by fours)
+    const int run_grid = ctx->sms * (4 / kEncJobsPerCta) *
+                         (int)(tail ? ctx->tune.enc_run_ctas_per_sm : ctx->tune.enc_run_ctas_per_sm_uniform);
     if (persistent) {
         cudaEvent_t t0;
         if (nlarge) {
@@ -171,7 +173,7 @@ int encode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
         }
         t0 = ctx->timer.begin(s);
         launch_enc_run(d_src, dB, dJ, (int)jobs.size(), dT, dW, queue, dK,
-                       std::min<int>(run_grid, (int)(jobs.size() + 3) / 4), s);
+                       std::min<int>(run_grid, (int)((jobs.size() + kEncJobsPerCta - 1) / kEncJobsPerCta)), s);
         ctx->timer.end(kStEncRun, t0, s);
     } else {
         // The plain form: every block gets its own launches, one after the other.

@@ -11,14 +11,6 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
     return m;
 }
 
-// Predicated stores: no branch, so unrolled rounds stay one basic block.
-__device__ __forceinline__ void st_u16_if(bool p, uint16_t *addr, uint32_t v) {
-    asm volatile(
-        "{\n .reg .pred q;\n setp.ne.b32 q, %0, 0;\n @q st.global.u16 [%1], %2;\n}" ::"r"((int)p), "l"(addr),
-        "h"((unsigned short)v)
-        : "memory");
-}
-
 __device__ __forceinline__ uint64_t warp_sum_u64(uint64_t v) {
 #pragma unroll
     for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -55,6 +47,66 @@ __device__ __forceinline__ uint64_t ld_u64_le(const uint8_t *p) {
 #pragma unroll
     for (int i = 7; i >= 0; i--) v = (v << 8) | p[i];
     return v;
+}
+
+// ---- encode table entries ---------------------------------------------------
+// The map of a state v below x_max = f << 20 (model.rs:125-133),
+//   x' = (v / f) 4096 + v % f + cum = v + cum + q (4096 - f),  q = v / f,
+// without a correction step: q is exact from one multiplication,
+//   q = hi32(v m + b m) >> s, b = 0 or 1.
+// For f not a power of two and 2^s < f: with m = ceil(2^(32+s) / f), b = 0
+// the product overshoots v / f by v (m f - 2^(32+s)) / (f 2^(32+s)), less
+// than the 1 / f it has to stay below, as v < 2^20 f, whenever f (m f -
+// 2^(32+s)) <= 2^(12+s) -- always for f < 2048; where it does not hold, the
+// floor with b = 1 does (its own remainder is then the smaller). A power of
+// two 2^k, k > 0, is m = 2^31, s = k - 1, and f = 1 takes q = v - 1 (m = 2^32
+// - 1, v > 0) with 4095 added to cum.
+// In the table arena an entry is 8 bytes:
+//   .m   m
+//   .y   (f - 1) << 20 | (cum, plus 4095 for f = 1) << 7 | b << 5 | s;
+//        0 for an absent symbol (no present one has 0).
+struct EncEntry {
+    uint32_t m, y;
+};
+__host__ __device__ inline EncEntry enc_entry_of(uint32_t f, uint32_t cum) {
+    if (f == 0) return {0u, 0u};
+    if (f == 1) return {0xffffffffu, (cum + 4095u) << 7};
+#ifdef __CUDA_ARCH__
+    const uint32_t s = 31u - (uint32_t)__clz((int)f);  // 2^s <= f < 2^(s+1)
+#else
+    uint32_t s = 0;
+    while ((2u << s) <= f) s++;
+#endif
+    if (f == 1u << s) return {0x80000000u, (f - 1u) << 20 | cum << 7 | (s - 1u)};
+    // 2^(32+s) = m f + r by 32-bit divisions: 2^32 = q f + r0 first
+    const uint32_t q = 0xffffffffu / f, r0 = 0xffffffffu - q * f + 1u;
+    const uint32_t t = (r0 << s) / f, r = (r0 << s) - t * f;
+    const uint32_t m = (q << s) + t, over = f - r;
+    const uint32_t b = f * over <= 4096u << s ? 0u : 1u;
+    return {m + 1u - b, (f - 1u) << 20 | cum << 7 | b << 5 | s};
+}
+// Frequency of an entry (0: absent).
+__host__ __device__ inline uint32_t enc_freq(uint32_t y) { return y ? (y >> 20) + 1u : 0u; }
+
+// The entry as the state's step takes it: a chain warp spends its time
+// issuing instructions, and this form leaves three to unpack it.
+struct EncStep {
+    uint32_t m;
+    uint32_t keep;  // largest state that keeps its low 16 bits, (f << 20) - 1
+    uint32_t pack;  // (cum, plus 4095 for f = 1) << 17 | (4096 - f) << 5 | s
+    uint32_t bias;  // b m
+};
+__host__ __device__ inline EncStep enc_unpack(uint32_t m, uint32_t y) {
+    return {m, y | 0xfffffu, ((y >> 7) & 0x1fffu) << 17 | (4095u - (y >> 20)) << 5 | (y & 31u), (y >> 5) & 1u ? m : 0u};
+}
+__host__ __device__ inline uint32_t enc_map(uint32_t v, const EncStep &e) {
+    const uint32_t hi = (uint32_t)(((uint64_t)v * e.m + e.bias) >> 32);
+#ifdef __CUDA_ARCH__
+    const uint32_t q = __funnelshift_r(hi, 0u, e.pack);  // by e.pack modulo 32: s
+#else
+    const uint32_t q = hi >> (e.pack & 31u);
+#endif
+    return v + (e.pack >> 17) + q * ((e.pack >> 5) & 0xfffu);
 }
 
 // Normalise m (<= 256) counts, held in ascending symbol order, into

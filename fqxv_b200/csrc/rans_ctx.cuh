@@ -129,11 +129,14 @@ struct Tuning {
     // table-image sizes cutting the other dense wide-alphabet streams into
     // launch groups (a launch's shared memory is its largest member's)
     int64_t dense_edge_small = 40 << 10, dense_edge_large = 80 << 10;
-    // encode kernel grid, CTAs per SM
-    int64_t enc_run_ctas_per_sm = 2;
-    // the same for batches of like-sized blocks (no block above four times
-    // the mean)
-    int64_t enc_run_ctas_per_sm_uniform = 3;
+    // Encode kernel grid, in jobs per SM counted by fours, for batches with a
+    // serial tail (a block above four times the mean): with more jobs beside
+    // them the largest run slower than the rest needs (2048 mixed blocks: 8.6
+    // ms at 1, 11.3 at 2) ...
+    int64_t enc_run_ctas_per_sm = 1;
+    // ... and for batches of like-sized blocks (2048 x 128 KiB: binned order-0
+    // 483 GB/s at 1, 706 at 2; full-range order-1 456 and 537; 2 is what fits).
+    int64_t enc_run_ctas_per_sm_uniform = 2;
     // Order-1 encode: 1, the model kernel stores each position's table index
     // (u16) for the encode kernel to read back; 0, the encode kernel derives
     // it from the byte and its predecessor (no per-position array).

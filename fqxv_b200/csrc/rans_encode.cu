@@ -5,7 +5,7 @@
 //      shared-memory atomics with run-length folding), exact normalisation,
 //      encode tables; for order-1 a dense |U| x |U| pair histogram and one
 //      normalised model per present context.
-//   2. enc_run_kernel     one warp per (block, order) job taken from a device
+//   2. enc_run_kernel     two warps per (block, order) job taken from a device
 //      work queue (jobs sorted largest first): lane l owns state l and walks
 //      the rounds from the last to the first, emitting renorm words with a
 //      ballot/popc compaction written back to front into a word scratch.
@@ -17,6 +17,7 @@
 #include <cooperative_groups.h>
 #include <mutex>
 
+#include "../../include/fqxv_rans_gpu_testing.h"
 #include "rans_common.cuh"
 #include "rans_internal.cuh"
 
@@ -82,11 +83,8 @@ __device__ __forceinline__ void histogram_pass(const uint8_t *__restrict__ p, ui
 }
 
 __device__ __forceinline__ uint2 enc_entry(uint32_t f, uint32_t cum) {
-    // avx2.rs:245-264: magic = floor((2^32 - 1) / f); fc = (f << 12) | cum.
-    // Absent symbols get an all-zero entry (their cum can be 4096, which
-    // would otherwise spill into the frequency field).
-    if (f == 0) return make_uint2(0u, 0u);
-    return make_uint2(0xffffffffu / f, (f << kScaleBits) | cum);
+    const EncEntry e = enc_entry_of(f, cum);
+    return make_uint2(e.m, e.y);
 }
 
 }  // namespace
@@ -252,297 +250,417 @@ __global__ void __launch_bounds__(kModelThreads)
 }
 
 // One encode step of a lane (scalar.rs:120-127 with the map of
-// model.rs:125-133, computed as avx2.rs:383-393): a state at or above
-// x_max = f << 20 gives up its low 16 bits (at most one word), then
-// x' = v + cum + q (4096 - f) with q = v / f from the magic reciprocal and one
-// correction. Both quotient candidates (with and without the renorm shift)
-// start at once, so the chain is compare -> select -> multiply -> compare ->
-// select. Returns whether the lane emits a word (its pre-step low 16 bits).
-__device__ __forceinline__ bool enc_step(uint32_t &x, uint2 e, bool active) {
-    const uint32_t f = e.y >> kScaleBits;
-    const uint32_t cum = e.y & (kTotFreq - 1);
-    const uint32_t xmax_m1 = (f << 20) - 1u;  // wraps to 2^32 - 1 for f == 4096: never emits
-    const uint32_t cmpl = kTotFreq - f;
-    const bool need = active && x > xmax_m1;
-    const uint32_t xs = x >> 16;
-    const uint32_t qa = __umulhi(x, e.x);
-    const uint32_t qb = __umulhi(xs, e.x);
-    const uint32_t v = need ? xs : x;
-    const uint32_t q0 = need ? qb : qa;
-    const uint32_t r0 = v - q0 * f;
-    const uint32_t x0 = v + cum + q0 * cmpl;
-    const uint32_t xn = r0 >= f ? x0 + cmpl : x0;
-    if (active) x = xn;
+// model.rs:125-133): a state at or above x_max = f << 20 gives up its low 16
+// bits (at most one word). Returns whether the lane emits a word (its pre-step
+// low 16 bits).
+__device__ __forceinline__ bool enc_step(uint32_t &x, const EncStep &e) {
+    const bool need = x > e.keep;
+    x = enc_map(need ? x >> 16 : x, e);
     return need;
 }
 
-// Emit the words of one round: the reference emits them high lane first
-// (scalar.rs:39-43), so stored below `wptr` they land in ascending lane order
-// and the finished region is already in decode order (scalar.rs:134-139).
-__device__ __forceinline__ void enc_emit(bool need, uint32_t word, uint16_t *__restrict__ &wptr, uint32_t lt) {
-    const uint32_t mask = __ballot_sync(0xffffffffu, need);
-    wptr -= __popc(mask);
-    st_u16_if(need, wptr + __popc(mask & lt), word);
+// Reverse-order encode of one block (scalar.rs:39-43 / :84-90) by two warps.
+// The states' chain is all that is serial; where each word goes is not. So a
+// chain warp (lane l owns state l, round r covers positions [32r, 32r + 32))
+// walks the rounds from the last to the first in chunks of kEncChunk, and
+// leaves each round's pre-step states and every lane's emit flags in shared
+// memory; an emit warp on another scheduler compacts the words of one chunk
+// (a vote and two population counts per round) while the chain runs the next.
+// Two message buffers per pair, a named barrier for each buffer and direction.
+//
+// Measured on B200, cycles per round of one stream (1 MiB): one warp doing
+// both, with a corrected reciprocal, 81 (order-0) and 86 (order-1); two warps
+// 57. Bulk (2048 x 128 KiB), GB/s of input: binned order-0 497 -> 708,
+// full-range order-1 476 -> 535, the latter at 88% of the shared-memory
+// wavefronts (12 a round, most of them 16-byte table entries).
+constexpr int kEncChunk = 16;
+
+struct EncMsg {
+    uint16_t word[kEncChunk][32];  // pre-step states' low halves, by round
+    uint32_t bits[32];             // lane's emit flags, bit k = round k of the chunk
+    int32_t job;                   // -1: no more jobs
+    int32_t flags;                 // 1: first chunk of the job, 2: last
+};
+
+// Message fields by 32-bit shared addresses (through a pointer kept in a
+// struct the compiler would take generic loads and stores).
+constexpr uint32_t kMsgBits = kEncChunk * 64, kMsgJob = kMsgBits + 128, kMsgBytes = kMsgJob + 8;
+static_assert(sizeof(EncMsg) == kMsgBytes, "message layout");
+__device__ __forceinline__ uint32_t lds_u16(uint32_t a) {
+    uint16_t v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint32_t lds_u32(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+// Table entries (the table was written before a __syncwarp): unpacked ones
+// of 16 bytes, and the arena's of 8.
+__device__ __forceinline__ EncStep lds_step(uint32_t a) {
+    EncStep e;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(e.m), "=r"(e.keep), "=r"(e.pack), "=r"(e.bias)
+                 : "r"(a));
+    return e;
+}
+__device__ __forceinline__ EncStep lds_entry(uint32_t a) {
+    uint32_t m, y;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(m), "=r"(y) : "r"(a));
+    return enc_unpack(m, y);
+}
+__device__ __forceinline__ void sts_u16(uint32_t a, uint32_t v) {
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((unsigned short)v));
+}
+__device__ __forceinline__ void sts_u32(uint32_t a, uint32_t v) {
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v));
 }
 
-// Reverse-order encode of one block by one warp (scalar.rs:39-43 / :84-90).
-// Lane l owns state l; round r covers positions [32r, 32r + 32). The partial
-// top round goes first, then the full rounds from the last to the first in
-// chunks of 16 whose symbols are loaded one chunk ahead. Word emission (a
-// warp vote per round) is kept off the state chain: a chunk records its
-// emit flags and pre-step states, and its words are written while the next
-// chunk's states are computed.
-template <int ORDER, bool SMEM_TAB, bool KEYS>
-__device__ __forceinline__ void encode_warp(const uint8_t *__restrict__ p, uint64_t n,
-                                            const uint2 *__restrict__ tab,
-                                            const uint8_t *__restrict__ umap, uint32_t nu,
-                                            const uint16_t *__restrict__ keys,
-                                            uint16_t *__restrict__ words, uint64_t word_end,
-                                            uint64_t &nwords, uint32_t &state) {
+// Barriers of pair p: 1 + 4 p + b when buffer b is full, + 2 when it is empty.
+struct WordPipe {
+    uint32_t msg;  // shared address of buffer 0
+    int id;
+    uint32_t sent;
+    __device__ WordPipe(EncMsg *m, int pair)
+        : msg((uint32_t)__cvta_generic_to_shared(m)), id(1 + 4 * pair), sent(0) {}
+    // The buffer of the next message, once the emit warp has read it.
+    __device__ __forceinline__ uint32_t open() {
+        if (sent >= 2) asm volatile("bar.sync %0, 64;" ::"r"(id + 2 + (int)(sent & 1)) : "memory");
+        return msg + (sent & 1) * kMsgBytes;
+    }
+    __device__ __forceinline__ void close(uint32_t m, uint32_t bits, int job, int flags) {
+        const uint32_t lane = threadIdx.x & 31;
+        sts_u32(m + kMsgBits + 4 * lane, bits);
+        if (lane == 0) {
+            sts_u32(m + kMsgJob, (uint32_t)job);
+            sts_u32(m + kMsgJob + 4, (uint32_t)flags);
+        }
+        __syncwarp();
+        asm volatile("bar.arrive %0, 64;" ::"r"(id + (int)(sent & 1)) : "memory");
+        sent++;
+    }
+    // The last message: no buffer is left in flight (one arrival of the emit
+    // warp, for the message before, is still to be taken).
+    __device__ void finish() {
+        close(open(), 0u, -1, 0);
+        if (sent >= 2) asm volatile("bar.sync %0, 64;" ::"r"(id + 2 + (int)(sent & 1)) : "memory");
+    }
+};
+
+// Emit warp: the words of every chunk of its pair's jobs, stored back to
+// front below the end of the job's region -- the reference emits them high
+// lane first (scalar.rs:39-43), so they land in ascending lane order and the
+// finished region is already in decode order (scalar.rs:134-139).
+__device__ __forceinline__ void emit_words(EncMsg *buffers, int pair, EncBlock *__restrict__ blocks,
+                                           const EncJob *__restrict__ jobs, uint16_t *__restrict__ words) {
+    const int lane = threadIdx.x & 31, id = 1 + 4 * pair;
+    const uint32_t ge = 0xffffffffu << lane;
+    const uint32_t msg = (uint32_t)__cvta_generic_to_shared(buffers);
+    uint16_t *end = nullptr, *wend = nullptr;
+    for (uint32_t b = 0;; b ^= 1u) {
+        asm volatile("bar.sync %0, 64;" ::"r"(id + (int)b) : "memory");
+        const uint32_t m = msg + b * kMsgBytes;
+        const int j = (int)lds_u32(m + kMsgJob);
+        if (j < 0) return;
+        const int flags = (int)lds_u32(m + kMsgJob + 4);
+        const uint32_t bits = lds_u32(m + kMsgBits + 4 * lane);
+        uint32_t w[kEncChunk];
+#pragma unroll
+        for (int k = 0; k < kEncChunk; k++) w[k] = lds_u16(m + 64 * k + 2 * lane);
+        if (flags & 1) {
+            const EncJob job = jobs[j];
+            end = wend = words + blocks[job.block].word_off[job.order] + blocks[job.block].n;
+        }
+        // at: the write position, in words from wend (below 0). One block of
+        // PTX per round, so that the vote and the store share a predicate.
+        int32_t at = 0;
+#pragma unroll
+        for (int k = 0; k < kEncChunk; k++)
+            asm volatile(
+                "{\n"
+                " .reg .pred q;\n"
+                " .reg .b32 t, v, c;\n"
+                " .reg .b64 a;\n"
+                " and.b32 t, %1, %5;\n"
+                " setp.ne.u32 q, t, 0;\n"
+                " vote.sync.ballot.b32 v, q, 0xffffffff;\n"
+                " and.b32 t, v, %2;\n"
+                " popc.b32 c, t;\n"
+                " sub.s32 c, %0, c;\n"
+                " mad.wide.s32 a, c, 2, %3;\n"
+                " @q st.global.u16 [a], %4;\n"
+                " popc.b32 c, v;\n"
+                " sub.s32 %0, %0, c;\n"
+                "}"
+                : "+r"(at)
+                : "r"(bits), "r"(ge), "l"(wend), "h"((unsigned short)w[k]), "r"(1u << k)
+                : "memory");
+        wend += at;
+        __syncwarp();
+        asm volatile("bar.arrive %0, 64;" ::"r"(id + 2 + (int)b) : "memory");
+        if ((flags & 2) && lane == 0) {
+            const EncJob job = jobs[j];
+            blocks[job.block].nwords[job.order] = (uint64_t)(end - wend);
+        }
+    }
+}
+
+// Symbols (or order-1 table indices) of the chunks ahead: a ring of kStages
+// chunks in shared memory filled by 16-byte asynchronous copies.
+constexpr int kStages = 4;
+template <class E>
+struct SymbolRing {
+    static constexpr uint32_t kBytes = kEncChunk * 32 * sizeof(E), kStage = kBytes + 16;
+    const uint8_t *top;  // address of the first element of chunk 0
+    uint32_t ring;       // shared address
+    uint32_t mis;        // its misalignment, the same for every chunk
+    int64_t chunks;
+
+    // `first`: element 0 of the block; chunk c holds the rounds
+    // [full - 16 (c + 1), full - 16 c).
+    __device__ SymbolRing(const E *first, int64_t full, uint32_t smem) {
+        chunks = full / kEncChunk;
+        top = reinterpret_cast<const uint8_t *>(first + (full - kEncChunk) * 32);
+        mis = (uint32_t)(uintptr_t)top & 15u;
+        top -= mis;
+        ring = smem;
+    }
+    __device__ __forceinline__ uint32_t stage(int64_t c) const { return ring + (uint32_t)(c & (kStages - 1)) * kStage; }
+    // Every copied granule of 16 bytes holds a byte of the chunk.
+    __device__ __forceinline__ void fetch(int64_t c) const {
+        const uint32_t lane = threadIdx.x & 31;
+        if (c < chunks) {
+            const uint8_t *g = top - c * (int64_t)kBytes;
+            const uint32_t d = stage(c);
+#pragma unroll
+            for (uint32_t o = 0; o < kBytes; o += 512)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + o + 16 * lane), "l"(g + o + 16 * lane));
+            if (lane == 0 && mis)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + kBytes), "l"(g + kBytes));
+        }
+        asm volatile("cp.async.commit_group;");
+    }
+    // Waits until at most LEFT of the fetched chunks are still on their way.
+    template <int LEFT>
+    static __device__ __forceinline__ void wait() {
+        asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
+        __syncwarp();
+    }
+    // Element of the chunk's k-th round from the top.
+    __device__ __forceinline__ uint32_t at(uint32_t s, int k) const {
+        const uint32_t a = s + mis + (uint32_t)sizeof(E) * (32 * (kEncChunk - 1 - k) + (threadIdx.x & 31));
+        if constexpr (sizeof(E) == 1) {
+            uint32_t v;
+            asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(a));
+            return v;
+        } else {
+            return lds_u16(a);
+        }
+    }
+};
+
+// Chain warp of one job. `first`: element 0 of the block (E: symbols, or
+// order-1 table indices); `entry(s, up)`: the table entry of element s. CTX
+// (order-1 on symbols): up is the context, byte i - 1 of position i, which
+// for lanes 1-31 is the symbol the lane below holds in the same round, and for
+// lane 0 the symbol lane 31 holds one round lower -- one shuffle per round
+// instead of a second load.
+template <bool CTX, class E, class Entry>
+__device__ __forceinline__ uint32_t encode_chain(uint64_t n, const E *__restrict__ first, Entry &&entry,
+                                                 WordPipe &pipe, int job, uint32_t ring) {
     const int lane = threadIdx.x & 31;
-    const uint32_t lt = lanemask_lt();
     uint32_t x = kRansL;
-    uint16_t *wptr = words + word_end;
     const int64_t full = (int64_t)(n / 32);
     const uint32_t rem = (uint32_t)(n % 32);
-    // Table entry of symbol s with predecessor `prev` (order-1: scalar.rs:85).
-    // With KEYS, `s` is already the position's order-1 table index.
-    auto entry = [&](uint32_t s, uint32_t prev) -> uint2 {
-        if (ORDER == 0) return tab[s];
-        const uint32_t idx = KEYS ? s : (uint32_t)umap[prev] * nu + umap[s];
-        return SMEM_TAB ? tab[idx] : __ldg(tab + idx);
-    };
-    // symbol (or table index) of position i, and its context byte
-    auto sym_at = [&](uint64_t i) -> uint32_t { return KEYS ? (uint32_t)keys[i] : (uint32_t)__ldg(p + i); };
-    constexpr bool CTX = ORDER == 1 && !KEYS;
+    auto sym = [&](uint64_t i) -> uint32_t { return (uint32_t)first[i]; };
+    const SymbolRing<E> R(first, full, ring);
+    __syncwarp();  // the last job's reads of the ring are done
+#pragma unroll
+    for (int c = 0; c < kStages - 1; c++) R.fetch(c);
+    int flags = 1;
     if (rem) {
         const uint64_t i = (uint64_t)full * 32 + lane;
         const bool active = lane < (int)rem;
-        const uint32_t s = active ? sym_at(i) : 0u;
-        uint32_t prev = 0;
-        if (CTX) prev = (active && i > 0) ? (uint32_t)__ldg(p + i - 1) : 0u;
-        const uint2 e = active ? entry(s, prev) : make_uint2(0u, 0u);
-        const uint32_t x_before = x;
-        const bool need = enc_step(x, e, active);
-        enc_emit(need, x_before, wptr, lt);
+        const uint32_t s = active ? sym(i) : 0u;
+        uint32_t up = 0;
+        if (CTX) up = active && i > 0 ? sym(i - 1) : 0u;
+        const uint32_t m = pipe.open();
+        sts_u16(m + 2 * lane, x);
+        const uint32_t bits = active && enc_step(x, entry(s, up)) ? 1u : 0u;
+        pipe.close(m, bits, job, full ? 1 : 3);
+        flags = 0;
     }
-    // cur/nxt: symbols of this chunk and the next; for order-1 also the
-    // byte before each position (its context, scalar.rs:85; 0 before the
-    // first byte), loaded with them instead of exchanged between lanes.
-    uint32_t cur[16], nxt[16], curp[16], nxtp[16], wv[16], pwv[16];
-    uint32_t pbits = 0;  // emit flags of the previous chunk (bit k = round rt + 16 - k)
+    const int64_t tail = full % kEncChunk;  // rounds below the whole chunks
+    // Symbols of chunk c, whose next chunk is on its way; past the whole
+    // chunks, of the rounds below them. `low`: the round below the lowest.
+    struct Symbols {
+        uint32_t s[kEncChunk], low;
+    };
+    auto look = [&](int64_t c, Symbols &S) {
+        S.low = 0;
+        if (c < R.chunks) {
+            // keyless order-1 also reads the top round of chunk c + 1
+            SymbolRing<E>::template wait<CTX ? 0 : 1>();
+            const uint32_t st = R.stage(c);
 #pragma unroll
-    for (int k = 0; k < 16; k++) {
-        const int64_t r = full - 1 - k;
-        const uint64_t i = (uint64_t)r * 32 + lane;
-        cur[k] = r >= 0 ? sym_at(i) : 0u;
-        curp[k] = (CTX && r >= 0 && i > 0) ? (uint32_t)__ldg(p + i - 1) : 0u;
-        pwv[k] = 0;
-    }
-    for (int64_t rt = full - 1; rt >= 0; rt -= 16) {
-        if (rt >= 32) {
-            const uint64_t ic = (uint64_t)(rt - 16) * 32 + lane;
-#pragma unroll
-            for (int k = 0; k < 16; k++) {
-                nxt[k] = sym_at(ic - 32 * k);
-                if (CTX) nxtp[k] = (uint32_t)__ldg(p + ic - 32 * k - 1);
-            }
+            for (int k = 0; k < kEncChunk; k++) S.s[k] = R.at(st, k);
+            if constexpr (CTX)
+                S.low = c + 1 < R.chunks ? R.at(R.stage(c + 1), 0) : tail ? sym((uint64_t)(tail - 1) * 32 + lane) : 0u;
         } else {
 #pragma unroll
-            for (int k = 0; k < 16; k++) {
-                const int64_t r = rt - 16 - k;
-                const uint64_t i = (uint64_t)r * 32 + lane;
-                nxt[k] = r >= 0 ? sym_at(i) : 0u;
-                nxtp[k] = (CTX && r >= 0 && i > 0) ? (uint32_t)__ldg(p + i - 1) : 0u;
-            }
-        }
-        const bool whole = rt >= 15;
-        // The chunk's table entries first: they depend only on the symbols,
-        // so their loads overlap one another instead of stalling the state
-        // chain one round at a time (a warp issues in order).
-        uint2 ent[16];
-#pragma unroll
-        for (int k = 0; k < 16; k++) ent[k] = entry(cur[k], CTX ? curp[k] : 0u);
-        uint32_t bits = 0;
-#pragma unroll
-        for (int k = 0; k < 16; k++) {
-            wv[k] = x;
-            const bool active = whole || k <= rt;
-            if (enc_step(x, ent[k], active)) bits |= 1u << k;
-            enc_emit((pbits >> k) & 1u, pwv[k], wptr, lt);
-        }
-        pbits = bits;
-#pragma unroll
-        for (int k = 0; k < 16; k++) {
-            cur[k] = nxt[k];
-            curp[k] = nxtp[k];
-            pwv[k] = wv[k];
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < 16; k++) enc_emit((pbits >> k) & 1u, pwv[k], wptr, lt);
-    nwords = (uint64_t)((words + word_end) - wptr);
-    state = x;
-}
-
-// Order-1 reverse encode without a per-position key array (scalar.rs:84-90):
-// the context of position i is byte i - 1, which for lanes 1-31 is the
-// symbol the lane below holds in the same round, and for lane 0 the symbol
-// lane 31 holds one round lower -- one shuffle per round instead of a second
-// byte load. A chunk's table entries (dense index of the context and the
-// symbol, then the table) are computed while the chunk above it runs its
-// state chain, from symbols loaded one chunk earlier (the byte below a
-// chunk's lowest round too), so neither the loads nor the lookups stand
-// between one chunk's chain and the next.
-template <bool SMEM_TAB>
-__device__ __forceinline__ void encode_warp_o1(const uint8_t *__restrict__ p, uint64_t n,
-                                               const uint2 *__restrict__ tab, const uint8_t *__restrict__ umap,
-                                               uint32_t nu, uint16_t *__restrict__ words, uint64_t word_end,
-                                               uint64_t &nwords, uint32_t &state) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t lt = lanemask_lt();
-    const uint32_t below = (uint32_t)(lane + 31) & 31u;  // the lane holding the byte before this lane's
-    uint32_t x = kRansL;
-    uint16_t *wptr = words + word_end;
-    const int64_t full = (int64_t)(n / 32);
-    const uint32_t rem = (uint32_t)(n % 32);
-    auto tabat = [&](uint32_t idx) -> uint2 { return SMEM_TAB ? tab[idx] : __ldg(tab + idx); };
-    auto sym = [&](int64_t r) -> uint32_t { return r >= 0 ? (uint32_t)__ldg(p + (uint64_t)r * 32 + lane) : 0u; };
-    if (rem) {
-        const uint64_t i = (uint64_t)full * 32 + lane;
-        const bool active = lane < (int)rem;
-        const uint32_t s = active ? (uint32_t)__ldg(p + i) : 0u;
-        const uint32_t prev = (active && i > 0) ? (uint32_t)__ldg(p + i - 1) : 0u;
-        const uint2 e = active ? tabat((uint32_t)umap[prev] * nu + umap[s]) : make_uint2(0u, 0u);
-        const uint32_t x_before = x;
-        const bool need = enc_step(x, e, active);
-        enc_emit(need, x_before, wptr, lt);
-    }
-    // entries of the chunk whose top round is rt, from its symbols cs[k]
-    // (round rt - k) and the symbol of round rt - 16 (lane 31's is the
-    // context of lane 0 in round rt - 15); rounds below 0 hold symbol 0,
-    // which is the context of position 0
-    auto entries = [&](const uint32_t (&cs)[16], uint32_t low, uint2 (&ent)[16]) {
-        uint32_t u[17];
-#pragma unroll
-        for (int k = 0; k < 16; k++) u[k] = umap[cs[k]];
-        u[16] = umap[low];
-#pragma unroll
-        for (int k = 0; k < 16; k++) {
-            const uint32_t up = __shfl_sync(0xffffffffu, lane == 31 ? u[k + 1] : u[k], below);
-            ent[k] = tabat(up * nu + u[k]);
+            for (int k = 0; k < kEncChunk; k++)
+                S.s[k] = c == R.chunks && k < tail ? sym((uint64_t)(tail - 1 - k) * 32 + lane) : 0u;
         }
     };
-    // c1: symbols of the chunk below the running one; lo1: the round below
-    // c1's lowest (its lane 31 holds the context of c1's lowest lane 0).
-    // Both are loaded one chunk before `entries` reads them.
-    uint32_t c1[16], c2[16], wv[16], pwv[16], lo1, lo2;
-    uint2 ent[16], entn[16];
-    uint32_t pbits = 0;
-#pragma unroll
-    for (int k = 0; k < 16; k++) {
-        c1[k] = sym(full - 1 - k);
-        pwv[k] = 0;
-    }
-    {
-        uint32_t c0[16];
-#pragma unroll
-        for (int k = 0; k < 16; k++) c0[k] = c1[k];
-#pragma unroll
-        for (int k = 0; k < 16; k++) c1[k] = sym(full - 17 - k);
-        lo1 = sym(full - 33);
-        entries(c0, c1[0], ent);
-    }
-    for (int64_t rt = full - 1; rt >= 0; rt -= 16) {
-#pragma unroll
-        for (int k = 0; k < 16; k++) c2[k] = sym(rt - 32 - k);
-        lo2 = sym(rt - 48);
-        entries(c1, lo1, entn);
-        const bool whole = rt >= 15;
+    auto step_of = [&](const Symbols &S, int k) {
+        uint32_t up = 0;
+        if constexpr (CTX) {
+            const uint32_t below = (uint32_t)(lane + 31) & 31u;
+            up = __shfl_sync(0xffffffffu, lane == 31 ? (k + 1 < kEncChunk ? S.s[(k + 1) % kEncChunk] : S.low) : S.s[k],
+                             below);
+        }
+        return entry(S.s[k], up);
+    };
+    // A round's table entry is loaded kAhead rounds before its step, across
+    // the chunks' edges (a ring of eight in registers), and a chunk's symbols
+    // one chunk before: loaded where they are used, they cost every chunk
+    // their latencies, about 240 cycles.
+    constexpr int kAhead = 6;
+    EncStep e[8];
+    auto chunk = [&](int64_t c, const Symbols &S, Symbols &N, uint32_t on, bool all) {
+        const bool last = c + 1 == R.chunks + (tail ? 1 : 0);
+        const uint32_t m = pipe.open(), mine = m + 2 * lane;
         uint32_t bits = 0;
 #pragma unroll
-        for (int k = 0; k < 16; k++) {
-            wv[k] = x;
-            const bool active = whole || k <= rt;
-            if (enc_step(x, ent[k], active)) bits |= 1u << k;
-            enc_emit((pbits >> k) & 1u, pwv[k], wptr, lt);
+        for (int k = 0; k < kEncChunk; k++) {
+            if (k == 2) {
+                // chunk c's stage was read a chunk ago; the chunk kStages - 1
+                // ahead takes the one before it
+                look(c + 1, N);
+                R.fetch(c + kStages - 1);
+            }
+            e[(k + kAhead) & 7] = k + kAhead < kEncChunk ? step_of(S, (k + kAhead) % kEncChunk)
+                                                         : step_of(N, (k + kAhead) % kEncChunk);
+            sts_u16(mine + 64 * k, x);
+            if (all || (on >> k) & 1u)
+                if (enc_step(x, e[k & 7])) bits |= 1u << k;
         }
-        pbits = bits;
+        pipe.close(m, bits, job, flags | (last ? 2 : 0));
+        flags = 0;
+    };
+    Symbols A, B;
+    look(0, A);
 #pragma unroll
-        for (int k = 0; k < 16; k++) {
-            ent[k] = entn[k];
-            c1[k] = c2[k];
-            pwv[k] = wv[k];
-        }
-        lo1 = lo2;
+    for (int k = 0; k < kAhead; k++) e[k] = step_of(A, k);
+    int64_t c = 0;
+    for (; c + 1 < R.chunks; c += 2) {
+        chunk(c, A, B, 0u, true);
+        chunk(c + 1, B, A, 0u, true);
     }
-#pragma unroll
-    for (int k = 0; k < 16; k++) enc_emit((pbits >> k) & 1u, pwv[k], wptr, lt);
-    nwords = (uint64_t)((words + word_end) - wptr);
-    state = x;
+    // at most one whole chunk and the rounds below
+    for (const int64_t end = R.chunks + (tail ? 1 : 0); c < end; c++) {
+        chunk(c, A, B, c < R.chunks ? 0xffffffffu : (1u << tail) - 1u, false);
+        A = B;
+    }
+    SymbolRing<E>::template wait<0>();
+    return x;
 }
 
-// Order-1 tables of alphabets up to kEncO1SmemNu symbols are copied into
-// the warp's slice of dynamic shared memory; larger ones are read through L1.
+// Order-1 tables are copied into the pair's slice of dynamic shared memory:
+// unpacked for alphabets of up to kEncO1StepNu symbols, as they are in the
+// arena for up to kEncO1SmemNu; larger ones are read through L1.
+constexpr uint32_t kEncO1StepNu = 32;
 constexpr uint32_t kEncO1SmemNu = 45;
-constexpr uint32_t kEncO1TabBytes = (kEncO1SmemNu * kEncO1SmemNu * 8 + 127) / 128 * 128;
+constexpr uint32_t kEncO1TabBytes = kEncO1StepNu * kEncO1StepNu * 16;
+static_assert(kEncO1SmemNu * kEncO1SmemNu * 8 <= kEncO1TabBytes, "a packed table fits the slice");
 
-__global__ void __launch_bounds__(kEncWarpsPerCta * 32)
+// Warps 0 .. kEncJobsPerCta - 1 are chain warps, the others emit warps, each
+// of the next pair's number, so a pair's two warps sit on two schedulers.
+__global__ void __launch_bounds__(kEncJobsPerCta * 64, 4)
     enc_run_kernel(const uint8_t *__restrict__ src, EncBlock *__restrict__ blocks,
                    const EncJob *__restrict__ jobs, int njobs, const uint8_t *__restrict__ tbl,
                    uint16_t *__restrict__ words, int *__restrict__ queue, const uint16_t *__restrict__ keys) {
     extern __shared__ __align__(16) uint8_t dsm[];
-    __shared__ uint2 s_tab[kEncWarpsPerCta][256];
-    __shared__ uint8_t s_umap[kEncWarpsPerCta][256];
+    __shared__ EncStep s_tab[kEncJobsPerCta][256];
+    __shared__ uint8_t s_umap[kEncJobsPerCta][256];
+    __shared__ __align__(16) EncMsg s_msg[kEncJobsPerCta][2];
+    __shared__ __align__(16) uint8_t s_ring[kEncJobsPerCta][kStages * SymbolRing<uint16_t>::kStage];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp >= kEncJobsPerCta) {
+        emit_words(s_msg[warp - kEncJobsPerCta], warp - kEncJobsPerCta, blocks, jobs, words);
+        return;
+    }
+    WordPipe pipe(s_msg[warp], warp);
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(s_ring[warp]);
     for (;;) {
         int j = 0;
         if (lane == 0) j = atomicAdd(queue, 1);
         j = __shfl_sync(0xffffffffu, j, 0);
-        if (j >= njobs) return;
+        if (j >= njobs) break;
         const EncJob job = jobs[j];
         EncBlock &B = blocks[job.block];
         const uint64_t n = B.n;
         const uint8_t *p = src + B.src_off;
         const uint8_t *T = tbl + B.tbl_off;
-        const uint64_t word_end = B.word_off[job.order] + n;
-        uint64_t nw = 0;
         uint32_t st = kRansL;
-        if (n) {
-            if (job.order == 0) {
-                const uint2 *T0 = reinterpret_cast<const uint2 *>(T + kTblO0);
+        if (n == 0) {
+            if (lane == 0) B.nwords[job.order] = 0;
+        } else if (job.order == 0) {
+            const uint2 *T0 = reinterpret_cast<const uint2 *>(T + kTblO0);
+            const uint32_t tab0 = (uint32_t)__cvta_generic_to_shared(s_tab[warp]);
 #pragma unroll
-                for (int k = 0; k < 8; k++) s_tab[warp][lane * 8 + k] = T0[lane * 8 + k];
-                __syncwarp();
-                encode_warp<0, true, false>(p, n, s_tab[warp], nullptr, 0, nullptr, words, word_end, nw, st);
-            } else {
+            for (int k = 0; k < 8; k++) s_tab[warp][lane + 32 * k] = enc_unpack(T0[lane + 32 * k].x, T0[lane + 32 * k].y);
+            __syncwarp();
+            st = encode_chain<false>(n, p, [&](uint32_t s, uint32_t) { return lds_step(tab0 + 16 * s); }, pipe, j, ring);
+        } else {
+            const uint32_t nu = (uint32_t)B.nu;
+            const uint2 *T1 = reinterpret_cast<const uint2 *>(T + kTblO1);
+            const uint16_t *kp = keys ? keys + ((uintptr_t)src & 15u) + B.src_off : nullptr;
+            const uint8_t *um = s_umap[warp];
+            if (!keys) {
 #pragma unroll
                 for (int k = 0; k < 8; k++) s_umap[warp][lane * 8 + k] = T[kTblUmap + lane * 8 + k];
-                const uint32_t nu = (uint32_t)B.nu;
-                const uint2 *T1 = reinterpret_cast<const uint2 *>(T + kTblO1);
-                if (nu <= kEncO1SmemNu) {
-                    uint2 *t = reinterpret_cast<uint2 *>(dsm + warp * kEncO1TabBytes);
-                    for (uint32_t i = lane; i < nu * nu; i += 32) t[i] = T1[i];
-                    __syncwarp();
-                    if (keys)
-                        encode_warp<1, true, true>(p, n, t, s_umap[warp], nu, keys + ((uintptr_t)src & 15u) + B.src_off, words,
-                                                   word_end, nw, st);
-                    else
-                        encode_warp_o1<true>(p, n, t, s_umap[warp], nu, words, word_end, nw, st);
-                } else {
-                    __syncwarp();
-                    if (keys)
-                        encode_warp<1, false, true>(p, n, T1, s_umap[warp], nu, keys + ((uintptr_t)src & 15u) + B.src_off, words,
-                                                    word_end, nw, st);
-                    else
-                        encode_warp_o1<false>(p, n, T1, s_umap[warp], nu, words, word_end, nw, st);
-                }
+            }
+            const uint32_t tab1 = (uint32_t)__cvta_generic_to_shared(dsm + warp * kEncO1TabBytes);
+            auto index = [&](uint32_t s, uint32_t c) { return (uint32_t)um[c] * nu + um[s]; };
+            auto global = [&](uint32_t i) {
+                const uint2 e = __ldg(T1 + i);
+                return enc_unpack(e.x, e.y);
+            };
+            if (nu <= kEncO1StepNu) {
+                EncStep *t = reinterpret_cast<EncStep *>(dsm + warp * kEncO1TabBytes);
+                for (uint32_t i = lane; i < nu * nu; i += 32) t[i] = enc_unpack(T1[i].x, T1[i].y);
+            } else if (nu <= kEncO1SmemNu) {
+                uint2 *t = reinterpret_cast<uint2 *>(dsm + warp * kEncO1TabBytes);
+                for (uint32_t i = lane; i < nu * nu; i += 32) t[i] = T1[i];
+            }
+            __syncwarp();
+            if (keys) {
+                if (nu <= kEncO1StepNu)
+                    st = encode_chain<false>(n, kp, [&](uint32_t s, uint32_t) { return lds_step(tab1 + 16 * s); }, pipe,
+                                             j, ring);
+                else if (nu <= kEncO1SmemNu)
+                    st = encode_chain<false>(n, kp, [&](uint32_t s, uint32_t) { return lds_entry(tab1 + 8 * s); }, pipe,
+                                             j, ring);
+                else
+                    st = encode_chain<false>(n, kp, [&](uint32_t s, uint32_t) { return global(s); }, pipe, j, ring);
+            } else {
+                if (nu <= kEncO1StepNu)
+                    st = encode_chain<true>(
+                        n, p, [&](uint32_t s, uint32_t c) { return lds_step(tab1 + 16 * index(s, c)); }, pipe, j, ring);
+                else if (nu <= kEncO1SmemNu)
+                    st = encode_chain<true>(
+                        n, p, [&](uint32_t s, uint32_t c) { return lds_entry(tab1 + 8 * index(s, c)); }, pipe, j, ring);
+                else
+                    st = encode_chain<true>(
+                        n, p, [&](uint32_t s, uint32_t c) { return global(index(s, c)); }, pipe, j, ring);
             }
         }
         B.states[job.order][lane] = st;
-        if (lane == 0) B.nwords[job.order] = nw;
         __syncwarp();
     }
+    pipe.finish();
 }
 
 __global__ void __launch_bounds__(1024)
@@ -651,7 +769,7 @@ __global__ void __launch_bounds__(kPackThreads)
         if (o == 0) {
             const uint2 *T0 = reinterpret_cast<const uint2 *>(T + kTblO0);
             for (int s = tid; s < 256; s += blockDim.x) {
-                const uint32_t f = T0[s].y >> kScaleBits;
+                const uint32_t f = enc_freq(T0[s].y);
                 d[off + 2 * s] = (uint8_t)f;
                 d[off + 2 * s + 1] = (uint8_t)(f >> 8);
             }
@@ -693,7 +811,7 @@ __global__ void __launch_bounds__(kPackThreads)
             for (int e = tid; e < K * 256; e += blockDim.x) {
                 const uint32_t u = um[rowctx[e >> 8]];
                 const uint32_t us = um[e & 255];
-                const uint32_t f = (full || us != 0xffu) ? (T1[(size_t)u * nu + us].y >> kScaleBits) : 0u;
+                const uint32_t f = (full || us != 0xffu) ? enc_freq(T1[(size_t)u * nu + us].y) : 0u;
                 d[off + 2 * (uint64_t)e] = (uint8_t)f;
                 d[off + 2 * (uint64_t)e + 1] = (uint8_t)(f >> 8);
             }
@@ -746,16 +864,16 @@ void launch_enc_run(const uint8_t *src, EncBlock *blocks, const EncJob *jobs, in
         std::lock_guard<std::mutex> lk(mu);
         if (dev >= 0 && dev < 256 && !done[dev]) {
             cudaFuncSetAttribute(enc_run_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(kEncWarpsPerCta * kEncO1TabBytes));
-            // three CTAs per SM (the register limit) need ~225 KB of shared memory
+                                 (int)(kEncJobsPerCta * kEncO1TabBytes));
+            // four CTAs per SM (the register limit) need ~170 KB of shared memory
             cudaFuncSetAttribute(enc_run_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  cudaSharedmemCarveoutMaxShared);
             cudaGetLastError();
             done[dev] = true;
         }
     }
-    enc_run_kernel<<<grid, kEncWarpsPerCta * 32, kEncWarpsPerCta * kEncO1TabBytes, s>>>(src, blocks, jobs, njobs,
-                                                                                       tbl, words, queue, keys);
+    enc_run_kernel<<<grid, kEncJobsPerCta * 64, kEncJobsPerCta * kEncO1TabBytes, s>>>(src, blocks, jobs, njobs, tbl,
+                                                                                     words, queue, keys);
 }
 
 void launch_enc_select_scan(EncBlock *blocks, int nblocks, uint64_t *total, cudaStream_t s) {
@@ -769,3 +887,12 @@ void launch_enc_pack(EncBlock *blocks, int nblocks, const uint8_t *tbl, const ui
 }
 
 }  // namespace fqxv
+
+extern "C" int fqxv_rans_test_enc_map(uint32_t f, uint32_t cum, const uint32_t *v, size_t n, uint32_t *out) {
+    if (f == 0 || f > fqxv::kTotFreq || (n && (!v || !out))) return FQXV_RANS_E_INVALID_ARG;
+    const fqxv::EncEntry e = fqxv::enc_entry_of(f, cum);
+    const fqxv::EncStep s = fqxv::enc_unpack(e.m, e.y);
+    if (fqxv::enc_freq(e.y) != f || s.keep != (f << 20) - 1u) return FQXV_RANS_E_INVALID_ARG;
+    for (size_t i = 0; i < n; i++) out[i] = fqxv::enc_map(v[i], s);
+    return FQXV_RANS_OK;
+}

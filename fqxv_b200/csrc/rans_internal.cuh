@@ -26,8 +26,7 @@ constexpr uint64_t kStatesBytes = 4 * kStates;
 constexpr int kModelThreads = 512;          // model kernel: threads per CTA
 constexpr int kModelCluster = 8;            // model kernel: CTAs (one cluster) per large block
 constexpr uint64_t kModelClusterMin = 256 << 10;  // smaller blocks get one CTA each
-constexpr int kEncWarpsPerCta = 4;          // encode: one warp per (block, order)
-constexpr int kDecWarpsPerCta = 4;          // decode: one warp per stream
+constexpr int kEncJobsPerCta = 2;           // encode: two warps per (block, order) job
 constexpr int kParseThreads = 256;          // decode header/table kernel
 constexpr int kPackThreads = 256;           // output compaction
 constexpr int kPackParts = 8;               // output compaction: CTAs per block
@@ -55,7 +54,7 @@ struct EncJob {
 };
 
 // Table arena layout per block (bytes from tbl_off):
-//   [0, 2048)               order-0: 256 x uint2 {magic, (freq << 12) | cum}
+//   [0, 2048)               order-0: 256 x uint2 (EncEntry, rans_common.cuh)
 //   [2048, 2048 + 256)      order-1: u8 dense index of each byte value (0xFF: not in U)
 //   [2304, ...)             order-1: nu x nu x uint2, row = context, column = symbol
 constexpr uint64_t kTblO0 = 0;

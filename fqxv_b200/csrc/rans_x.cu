@@ -328,24 +328,16 @@ __global__ void __launch_bounds__(128) x_n4_run_kernel(const uint8_t *__restrict
     // one position of lane's state: emits the pre-step low 16 bits when the
     // state would pass x_max = f << 20 (never for f = 4096)
     auto step = [&](uint2 e, bool active) {
-        const uint32_t f = e.y >> kScaleBits, cum = e.y & (kTotFreq - 1);
         uint32_t v = x;
-        const bool need = active && (uint64_t)v >= ((uint64_t)f << 20);
+        const EncStep st = enc_unpack(e.x, e.y);
+        const bool need = active && v > st.keep;
         const uint32_t mask = __ballot_sync(0xffffffffu, need);
         w -= __popc(mask);
         if (need) {
             w[__popc(mask & lt)] = (uint16_t)v;
             v >>= 16;
         }
-        if (active) {
-            uint32_t q = __umulhi(v, e.x);
-            uint32_t r = v - q * f;
-            if (r >= f) {
-                q++;
-                r -= f;
-            }
-            x = (q << kScaleBits) + r + cum;
-        }
+        if (active) x = enc_map(v, st);
     };
     const uint64_t full = n / 4;
     const uint32_t rem = (uint32_t)(n % 4);
@@ -390,7 +382,7 @@ __global__ void __launch_bounds__(256) x_n4_pack_kernel(const EncBlock *__restri
         if (o == 0) {
             const uint2 *T0 = reinterpret_cast<const uint2 *>(T + kTblO0);
             for (int s = tid; s < 256; s += blockDim.x) {
-                const uint32_t f = T0[s].y >> kScaleBits;
+                const uint32_t f = enc_freq(T0[s].y);
                 d[off + 2 * s] = (uint8_t)f;
                 d[off + 2 * s + 1] = (uint8_t)(f >> 8);
             }
@@ -428,7 +420,7 @@ __global__ void __launch_bounds__(256) x_n4_pack_kernel(const EncBlock *__restri
             for (int e = tid; e < K * 256; e += blockDim.x) {
                 const uint32_t u = um[rowctx[e >> 8]];
                 const uint32_t us = um[e & 255];
-                const uint32_t f = (full || us != 0xffu) ? (T1[(size_t)u * nu + us].y >> kScaleBits) : 0u;
+                const uint32_t f = (full || us != 0xffu) ? enc_freq(T1[(size_t)u * nu + us].y) : 0u;
                 d[off + 2 * (uint64_t)e] = (uint8_t)f;
                 d[off + 2 * (uint64_t)e + 1] = (uint8_t)(f >> 8);
             }

@@ -8,6 +8,7 @@
 #ifndef FQXV_RANS_GPU_TESTING_H
 #define FQXV_RANS_GPU_TESTING_H
 
+#include <stddef.h>
 #include <stdint.h>
 
 #include "fqxv_rans_gpu.h"
@@ -25,6 +26,12 @@ extern "C" {
  * order-1 decoders reports FQXV_RANS_E_TIMEOUT while its copy still lands.
  * Applies to the context and its sub-contexts. */
 int fqxv_rans_ctx_test_set_wait_polls(fqxv_rans_ctx *ctx, uint32_t polls);
+
+/* The encoder's state map for a symbol of frequency f (1..4096) and cumulative
+ * frequency cum: out[i] = (v[i] / f) * 4096 + v[i] % f + cum, from the table
+ * entry's multiplication. Host arithmetic, the same functions as the kernels'.
+ * FQXV_RANS_E_INVALID_ARG when the entry does not give back f and f << 20. */
+int fqxv_rans_test_enc_map(uint32_t f, uint32_t cum, const uint32_t *v, size_t n, uint32_t *out);
 
 #ifdef __cplusplus
 }
