@@ -40,18 +40,24 @@ def _codec(device: int):
 
 
 def _spans(lens) -> np.ndarray:
-    lens = np.asarray(lens, dtype=np.uint64)
-    offs = np.zeros(len(lens), dtype=np.uint64)
-    if len(lens):
-        offs[1:] = np.cumsum(lens)[:-1]
-    return np.ascontiguousarray(np.stack([offs, lens], axis=1)) if len(lens) else np.zeros((0, 2), np.uint64)
+    """(offset, length) of items laid back to back; lens: any sized iterable
+    of ints."""
+    out = np.zeros((len(lens), 2), dtype=np.uint64)
+    out[:, 1] = lens if isinstance(lens, np.ndarray) else np.fromiter(lens, dtype=np.uint64, count=len(lens))
+    if len(out):
+        np.cumsum(out[:-1, 1], out=out[1:, 0])
+    return out
+
+
+def _lens(items) -> np.ndarray:
+    return np.fromiter(map(len, items), dtype=np.uint64, count=len(items))
 
 
 def encode_blocks(blocks, device: int = 0) -> list[bytes]:
     """One payload per block of names (each a list of bytes-like names)."""
-    names = [bytes(n) for blk in blocks for n in blk]
+    names = [n if type(n) is bytes else bytes(n) for blk in blocks for n in blk]
     arena = np.frombuffer(b"".join(names) or b"\0", dtype=np.uint8)
-    nsp = _spans([len(n) for n in names])
+    nsp = _spans(_lens(names))
     counts = [len(blk) for blk in blocks]
     bsp = _spans(counts)
     c = _codec(device)
@@ -60,7 +66,7 @@ def encode_blocks(blocks, device: int = 0) -> list[bytes]:
     need = ctypes.c_uint64(0)
     cap = 4 * arena.size + 4096 * len(blocks) + (1 << 16)
     for _ in range(2):
-        dst = np.zeros(max(cap, 1), dtype=np.uint8)
+        dst = np.empty(max(cap, 1), dtype=np.uint8)
         st = L.fqxv_tok_encode_host(c._h, arena.ctypes.data, nsp.ctypes.data, len(names), bsp.ctypes.data,
                                     len(blocks), dst.ctypes.data, dst.size, out.ctypes.data, ctypes.byref(need))
         if st == 17 and need.value > cap:
@@ -76,17 +82,21 @@ def decode_blocks(payloads, device: int = 0, raise_on_error: bool = True):
     statuses) with an empty list for a failed block."""
     payloads = [bytes(p) for p in payloads]
     arena = np.frombuffer(b"".join(payloads) or b"\0", dtype=np.uint8)
-    psp = _spans([len(p) for p in payloads])
+    psp = _spans(_lens(payloads))
     n = len(payloads)
     c = _codec(device)
     L = rans.lib()
     blocks = np.zeros((max(n, 1), 2), dtype=np.uint64)
     status = np.zeros(max(n, 1), dtype=np.int32)
     nb, ns = ctypes.c_uint64(0), ctypes.c_uint64(0)
-    names_cap, spans_cap = 8 * arena.size + 4096, arena.size + 64
+    # Untouched memory costs nothing; a buffer that turns out too small costs
+    # a second decode (sequencer names shrink 10 to 20 times). Large calls
+    # start from less.
+    names_cap = min(64 * arena.size, max(8 * arena.size, 1 << 28)) + 4096
+    spans_cap = min(4 * arena.size, max(arena.size, 1 << 24)) + 64
     for _ in range(2):
-        h_names = np.zeros(max(names_cap, 1), dtype=np.uint8)
-        nsp = np.zeros((max(spans_cap, 1), 2), dtype=np.uint64)
+        h_names = np.empty(max(names_cap, 1), dtype=np.uint8)
+        nsp = np.empty((max(spans_cap, 1), 2), dtype=np.uint64)
         st = L.fqxv_tok_decode_host(c._h, arena.ctypes.data, psp.ctypes.data, n, h_names.ctypes.data, names_cap,
                                     nsp.ctypes.data, spans_cap, blocks.ctypes.data, status.ctypes.data,
                                     ctypes.byref(nb), ctypes.byref(ns))
@@ -96,10 +106,14 @@ def decode_blocks(payloads, device: int = 0, raise_on_error: bool = True):
         break
     if st and st not in TOK_STATUSES and st not in rans.MALFORMED:
         _raise(st)
+    # One bytes object, sliced by plain ints: a numpy slice and copy per name
+    # took most of a call (128,000 names).
+    text = h_names[:nb.value].tobytes()
     out = []
     for b in range(n):
         f, k = int(blocks[b, 0]), int(blocks[b, 1])
-        out.append([h_names[int(o):int(o + l)].tobytes() for o, l in nsp[f:f + k]])
+        at = nsp[f:f + k, 0]
+        out.append([text[i:j] for i, j in zip(at.tolist(), (at + nsp[f:f + k, 1]).tolist())])
     if raise_on_error:
         for s in status[:n]:
             if s:
