@@ -1,10 +1,11 @@
 // Encode path of the B200 rANS Nx16 coder.
 //
 // Stages (each one launch over the whole batch):
-//   1. enc_model_kernel   one CTA per block: order-0 histogram (warp-private
-//      shared-memory atomics with run-length folding), exact normalisation,
-//      encode tables; for order-1 a dense |U| x |U| pair histogram and one
-//      normalised model per present context.
+//   1. enc_model_kernel   a cluster of CTAs per block: order-0 histogram (warp-
+//      private shared-memory atomics with run-length folding), exact
+//      normalisation, encode tables; for order-1 the occurring bytes, then a
+//      dense |U| x |U| pair histogram (whose column sums are the order-0
+//      counts) and one normalised model per present context.
 //   2. enc_run_kernel     two warps per (block, order) job taken from a device
 //      work queue (jobs sorted largest first): lane l owns state l and walks
 //      the rounds from the last to the first, emitting renorm words with a
@@ -82,6 +83,30 @@ __device__ __forceinline__ void histogram_pass(const uint8_t *__restrict__ p, ui
     }
 }
 
+// Marks the bytes that occur in positions [lo, hi) of p: plain byte stores,
+// which lanes with the same or neighbouring symbols share, where a count
+// takes an atomic per byte and serialises on equal ones (1 shared-memory
+// wavefront per 32 bytes against 4).
+__device__ __forceinline__ void seen_pass(const uint8_t *__restrict__ p, uint64_t lo, uint64_t hi,
+                                          volatile uint8_t *seen) {
+    if (hi <= lo) return;
+    const uint64_t n = hi - lo;
+    const uint64_t mis = (uint64_t)(uintptr_t)(p + lo) & 15u;
+    uint64_t head = mis ? 16 - mis : 0;
+    if (head > n) head = n;
+    const uint64_t body = (n - head) / 16;
+    for (uint64_t i = lo + threadIdx.x; i < lo + head; i += blockDim.x) seen[p[i]] = 1;
+    for (uint64_t i = lo + head + body * 16 + threadIdx.x; i < hi; i += blockDim.x) seen[p[i]] = 1;
+    const uint4 *q = reinterpret_cast<const uint4 *>(p + lo + head);
+    for (uint64_t c = threadIdx.x; c < body; c += blockDim.x) {
+        uint32_t b[16];
+        unpack16(__ldg(q + c), b);
+#pragma unroll
+        for (int k = 0; k < 16; k++)
+            if (k == 0 || b[k] != b[k - 1]) seen[b[k]] = 1;
+    }
+}
+
 __device__ __forceinline__ uint2 enc_entry(uint32_t f, uint32_t cum) {
     const EncEntry e = enc_entry_of(f, cum);
     return make_uint2(e.m, e.y);
@@ -104,6 +129,8 @@ __global__ void __launch_bounds__(kModelThreads)
     __shared__ uint32_t h1[kSmemU * kSmemU];
     __shared__ uint32_t part[256];      // this CTA's order-0 counts
     __shared__ uint32_t cnt[256];       // the block's order-0 counts
+    __shared__ uint32_t occurs[256];    // order-1: bytes of this CTA's slice
+    __shared__ uint8_t seen[256];
     __shared__ uint32_t rowbuf[W][kSmemU];
     __shared__ uint8_t umap[256];
     __shared__ int s_nu, s_nctx;
@@ -121,51 +148,72 @@ __global__ void __launch_bounds__(kModelThreads)
         uint8_t *T = tbl + blocks[b].tbl_off;
         const uint64_t lo = n * (uint64_t)rank / C, hi = n * (uint64_t)(rank + 1) / C;
 
-        for (int i = tid; i < W * 256; i += blockDim.x) (&h0[0][0])[i] = 0;
         if (tid == 0) s_nctx = 0;
-        __syncthreads();
-        uint32_t *hw = h0[warp];
-        histogram_pass(
-            p, lo, hi, [](uint32_t, uint32_t c) { return c; },
-            [&](uint32_t k, uint32_t r) { atomicAdd(&hw[k], r); }, [](uint64_t, uint32_t) {},
-            [](uint64_t, const uint32_t *) {});
-        __syncthreads();
-        if (tid < 256) {
-            uint32_t t = 0;
+        // order-0 counts of this CTA's slice in `part`, then of the block in
+        // `cnt`, and the order-0 table from them
+        auto count_slice = [&] {
+            for (int i = tid; i < W * 256; i += blockDim.x) (&h0[0][0])[i] = 0;
+            __syncthreads();
+            uint32_t *hw = h0[warp];
+            histogram_pass(
+                p, lo, hi, [](uint32_t, uint32_t c) { return c; },
+                [&](uint32_t k, uint32_t r) { atomicAdd(&hw[k], r); }, [](uint64_t, uint32_t) {},
+                [](uint64_t, const uint32_t *) {});
+            __syncthreads();
+            if (tid < 256) {
+                uint32_t t = 0;
 #pragma unroll
-            for (int w = 0; w < W; w++) t += h0[w][tid];
-            part[tid] = t;
-        }
-        cl.sync();  // every slice's counts are in place
-        if (tid < 256) {
-            uint32_t t = 0;
-            for (int r = 0; r < C; r++) t += cl.map_shared_rank(part, r)[tid];
-            cnt[tid] = t;
-        }
-        __syncthreads();
-
-        if (mode != FQXV_RANS_ORDER1 && rank == 0 && warp == 0) {
+                for (int w = 0; w < W; w++) t += h0[w][tid];
+                part[tid] = t;
+            }
+        };
+        auto sum_slices = [&] {
+            if (tid < 256) {
+                uint32_t t = 0;
+                for (int r = 0; r < C; r++) t += cl.map_shared_rank(part, r)[tid];
+                cnt[tid] = t;
+            }
+            __syncthreads();
+        };
+        auto order0_table = [&] {
+            if (rank != 0 || warp != 0) return;
             uint32_t f[8], cum[8];
             bool present;
             warp_normalize(cnt, 256, f, cum, present);
             uint2 *T0 = reinterpret_cast<uint2 *>(T + kTblO0);
 #pragma unroll
             for (int k = 0; k < 8; k++) T0[lane * 8 + k] = enc_entry(f[k], cum[k]);
-        }
+        };
         if (mode == FQXV_RANS_ORDER0) {
+            count_slice();
+            cl.sync();  // every slice's counts are in place
+            sum_slices();
+            order0_table();
             cl.sync();  // no CTA rewrites `part` while another still reads it
             continue;
         }
 
         // Order-1 (scalar.rs:62-80). U = occurring bytes plus context 0, in
         // ascending byte order; contexts and symbols share that dense index.
-        // Every CTA derives the same map from the same counts.
+        // Every CTA derives the same map from the same marks.
+        if (tid < 256) seen[tid] = 0;
+        __syncthreads();
+        seen_pass(p, lo, hi, seen);
+        __syncthreads();
+        if (tid < 256) occurs[tid] = seen[tid];
+        cl.sync();
+        if (tid < 256) {
+            uint32_t t = 0;
+            for (int r = 0; r < C; r++) t |= cl.map_shared_rank(occurs, r)[tid];
+            seen[tid] = (uint8_t)t;
+        }
+        __syncthreads();
         if (warp == 0) {
             uint32_t flags = 0;
 #pragma unroll
             for (int k = 0; k < 8; k++) {
                 const int s = lane * 8 + k;
-                if (cnt[s] != 0 || s == 0) flags |= 1u << k;
+                if (seen[s] != 0 || s == 0) flags |= 1u << k;
             }
             const uint32_t c = __popc(flags);
             uint32_t base = warp_incl_scan(c) - c;
@@ -200,7 +248,23 @@ __global__ void __launch_bounds__(kModelThreads)
             for (int i = tid; i < nu * nu; i += blockDim.x) h1[i] = 0;
             __syncthreads();
             histogram_pass(p, lo, hi, pair, [&](uint32_t k, uint32_t r) { atomicAdd(&h1[k], r); }, emit, emit16);
+            // every position is counted in one pair, so a symbol's order-0
+            // count is its column's sum
+            if (mode != FQXV_RANS_ORDER1) {
+                __syncthreads();
+                if (tid < 256) {
+                    const uint32_t u = umap[tid];
+                    uint32_t t = 0;
+                    if (u != 0xffu)
+                        for (int r = 0; r < nu; r++) t += h1[r * nu + u];
+                    part[tid] = t;
+                }
+            }
             cl.sync();
+            if (mode != FQXV_RANS_ORDER1) {
+                sum_slices();
+                order0_table();
+            }
             for (int t = warp + W * rank; t < nu; t += W * C) {
                 for (int u = lane; u < nu; u += 32) {
                     uint32_t v = 0;
@@ -219,23 +283,31 @@ __global__ void __launch_bounds__(kModelThreads)
                 if (lane == 0 && present) atomicAdd(&s_nctx, 1);
                 __syncwarp();
             }
-        } else if (rank == 0) {
+        } else {
+            if (mode != FQXV_RANS_ORDER1) {
+                count_slice();
+                cl.sync();
+                sum_slices();
+                order0_table();
+            }
             // large alphabets: the cluster's first CTA counts the whole block
             // in global scratch
-            for (int i = tid; i < nu * nu; i += blockDim.x) gh[i] = 0;
-            __syncthreads();
-            histogram_pass(p, 0, n, pair, [&](uint32_t k, uint32_t r) { atomicAdd(&gh[k], r); }, emit, emit16);
-            __syncthreads();
-            for (int t = warp; t < nu; t += W) {
-                uint32_t f[8], cum[8];
-                bool present;
-                warp_normalize(gh + (size_t)t * nu, nu, f, cum, present);
-#pragma unroll
-                for (int k = 0; k < 8; k++) {
-                    const int u = lane * 8 + k;
-                    if (u < nu) T1[(size_t)t * nu + u] = enc_entry(f[k], cum[k]);
+            if (rank == 0) {
+                for (int i = tid; i < nu * nu; i += blockDim.x) gh[i] = 0;
+                __syncthreads();
+                histogram_pass(p, 0, n, pair, [&](uint32_t k, uint32_t r) { atomicAdd(&gh[k], r); }, emit, emit16);
+                __syncthreads();
+                for (int t = warp; t < nu; t += W) {
+                    uint32_t f[8], cum[8];
+                    bool present;
+                    warp_normalize(gh + (size_t)t * nu, nu, f, cum, present);
+    #pragma unroll
+                    for (int k = 0; k < 8; k++) {
+                        const int u = lane * 8 + k;
+                        if (u < nu) T1[(size_t)t * nu + u] = enc_entry(f[k], cum[k]);
+                    }
+                    if (lane == 0 && present) atomicAdd(&s_nctx, 1);
                 }
-                if (lane == 0 && present) atomicAdd(&s_nctx, 1);
             }
         }
         cl.sync();  // all rows done; s_nctx final in every CTA
@@ -735,13 +807,16 @@ __device__ __forceinline__ void cta_copy(uint8_t *__restrict__ dst, const uint8_
     if (tid < hi - t) dst[t + tid] = src[t + tid];
 }
 
-// One work item per (block, part): part 0 writes the header, tables and
-// states, and every part copies its slice of the renorm words.
+// One work item per (block, part): part 0 writes the header and states, and
+// every part its share of the order-1 tables and of the renorm words (all
+// tables by part 0 kept its CTA busy long after the others: 2048 x 128 KiB
+// full-range blocks, 32 tables each, 376 us against 278).
 __global__ void __launch_bounds__(kPackThreads)
     enc_pack_kernel(const EncBlock *__restrict__ blocks, int nblocks, const uint8_t *__restrict__ tbl,
                     const uint16_t *__restrict__ words, uint8_t *__restrict__ dst) {
     __shared__ uint8_t present[256];
     __shared__ uint8_t rowctx[256];
+    __shared__ uint8_t s_um[256];
     __shared__ int s_k;
     const int tid = threadIdx.x;
     const int nitems = nblocks * kPackParts;
@@ -752,42 +827,37 @@ __global__ void __launch_bounds__(kPackThreads)
         const uint64_t n = B.n;
         uint8_t *d = dst + B.out_off;
         if (n == 0 && part != 0) continue;
-        const uint64_t hdr = o == 0 ? kHdr + kO0Tables : kHdr + kO1Bitmap + kO1Table * (uint64_t)B.nctx;
-        if (part != 0) {
-            const uint64_t W2 = 2 * B.nwords[o];
-            const uint64_t lo = (W2 * part / kPackParts) & ~(uint64_t)15;
-            const uint64_t hi = part + 1 == kPackParts ? W2 : (W2 * (part + 1) / kPackParts) & ~(uint64_t)15;
-            const uint8_t *ws = reinterpret_cast<const uint8_t *>(words + B.word_off[o] + n - B.nwords[o]);
-            cta_copy(d + hdr + kStatesBytes, ws, lo, hi);
-            continue;
+        if (part == 0) {
+            if (tid == 0) d[0] = (uint8_t)o;
+            if (tid >= 1 && tid <= 8) d[tid] = (uint8_t)(n >> (8 * (tid - 1)));
+            if (n == 0) continue;
         }
-        if (tid == 0) d[0] = (uint8_t)o;
-        if (tid >= 1 && tid <= 8) d[tid] = (uint8_t)(n >> (8 * (tid - 1)));
-        if (n == 0) continue;
         const uint8_t *T = tbl + B.tbl_off;
         uint64_t off = kHdr;
         if (o == 0) {
-            const uint2 *T0 = reinterpret_cast<const uint2 *>(T + kTblO0);
-            for (int s = tid; s < 256; s += blockDim.x) {
-                const uint32_t f = enc_freq(T0[s].y);
-                d[off + 2 * s] = (uint8_t)f;
-                d[off + 2 * s + 1] = (uint8_t)(f >> 8);
+            if (part == 0) {
+                const uint2 *T0 = reinterpret_cast<const uint2 *>(T + kTblO0);
+                for (int s = tid; s < 256; s += blockDim.x) {
+                    const uint32_t f = enc_freq(T0[s].y);
+                    d[off + 2 * s] = (uint8_t)f;
+                    d[off + 2 * s + 1] = (uint8_t)(f >> 8);
+                }
             }
             off += kO0Tables;
         } else {
             // scalar.rs:96-107: presence bitmap, then one table per present
             // context in ascending context order.
             const int nu = B.nu;
-            const uint8_t *um = T + kTblUmap;
             const uint2 *T1 = reinterpret_cast<const uint2 *>(T + kTblO1);
             // With all 256 byte values in U the map is the identity and 0xFF
             // is a real index, not the "absent" marker.
             const bool full = nu == 256;
             if (tid < 256) {
-                const uint32_t u = um[tid];
+                const uint32_t u = T[kTblUmap + tid];
                 bool pr = false;
                 if (full || u != 0xffu)
                     for (int v = 0; v < nu && !pr; v++) pr = T1[(size_t)u * nu + v].y != 0;
+                s_um[tid] = (uint8_t)u;
                 present[tid] = pr;
             }
             __syncthreads();
@@ -798,7 +868,7 @@ __global__ void __launch_bounds__(kPackThreads)
                     bits |= (uint32_t)present[tid * 8 + k] << k;
                     cntp += present[tid * 8 + k];
                 }
-                d[off + tid] = (uint8_t)bits;
+                if (part == 0) d[off + tid] = (uint8_t)bits;
                 uint32_t base = warp_incl_scan(cntp) - cntp;
 #pragma unroll
                 for (int k = 0; k < 8; k++)
@@ -808,25 +878,27 @@ __global__ void __launch_bounds__(kPackThreads)
             __syncthreads();
             off += kO1Bitmap;
             const int K = s_k;
-            for (int e = tid; e < K * 256; e += blockDim.x) {
-                const uint32_t u = um[rowctx[e >> 8]];
-                const uint32_t us = um[e & 255];
+            const int e1 = K * 256 * (part + 1) / kPackParts;
+            for (int e = K * 256 * part / kPackParts + tid; e < e1; e += blockDim.x) {
+                const uint32_t u = s_um[rowctx[e >> 8]];
+                const uint32_t us = s_um[e & 255];
                 const uint32_t f = (full || us != 0xffu) ? enc_freq(T1[(size_t)u * nu + us].y) : 0u;
                 d[off + 2 * (uint64_t)e] = (uint8_t)f;
                 d[off + 2 * (uint64_t)e + 1] = (uint8_t)(f >> 8);
             }
             off += kO1Table * (uint64_t)K;
         }
-        if (tid < kStates) {
+        if (part == 0 && tid < kStates) {
             const uint32_t x = B.states[o][tid];
 #pragma unroll
             for (int k = 0; k < 4; k++) d[off + 4 * tid + k] = (uint8_t)(x >> (8 * k));
         }
-        off += kStatesBytes;
         const uint64_t W2 = 2 * B.nwords[o];
+        const uint64_t lo = (W2 * part / kPackParts) & ~(uint64_t)15;
+        const uint64_t hi = part + 1 == kPackParts ? W2 : (W2 * (part + 1) / kPackParts) & ~(uint64_t)15;
         const uint8_t *ws = reinterpret_cast<const uint8_t *>(words + B.word_off[o] + n - B.nwords[o]);
-        cta_copy(d + off, ws, 0, kPackParts == 1 ? W2 : (W2 / kPackParts) & ~(uint64_t)15);
-        __syncthreads();
+        cta_copy(d + off + kStatesBytes, ws, lo, hi);
+        __syncthreads();  // the next item rewrites the shared arrays
     }
 }
 
