@@ -540,6 +540,17 @@ struct WordRing {
             __syncwarp();
         }
     }
+    // The same between groups of rounds, where the position has moved by a few
+    // segments at most: 32-bit arithmetic, and one test when nothing is due.
+    __device__ __forceinline__ void follow(uint32_t w32) {
+        while ((int32_t)(lead + w32 - kSegWords * (next_seg - 3)) >= 0) {
+            __syncwarp();
+            put(next_seg, pend, pend_next);
+            next_seg++;
+            fetch(next_seg, pend, pend_next);
+            __syncwarp();
+        }
+    }
     // Word j of the region; only the low bits of j matter (the ring is a
     // power-of-two window), so 32-bit arithmetic is exact here.
     __device__ __forceinline__ Elem at(uint32_t j) const { return ring[(lead + j) & (kRingWords - 1)]; }
@@ -723,50 +734,51 @@ __global__ void __launch_bounds__(32, 1)
         // renormalises takes them through one shuffle each from lane
         // popc(earlier needs), so the table lookup is off the round's
         // critical path. The next window is loaded as soon as the round's
-        // vote is known.
-        uint2 W = make_uint2(0, 0);
-        uint32_t e = 0;
-        bool window = false;
+        // vote is known. Groups are counted ahead and the ring follows with
+        // 32-bit arithmetic: one stream 129 cycles per round against 141 with
+        // the 64-bit checks between groups (256 KiB of binned quality).
         uint64_t r = 0;
-        if (rounds && !o0_general_round(x, P, 0, n, R, wp, navail, out, lt)) status = FQXV_RANS_E_TRUNCATED;
-        r = 1;
         constexpr int G = 8;  // rounds per branch-free group
         static_assert(32 * G + 64 <= 3 * kSegWords, "a group's words are resident after one ring advance");
         while (status == FQXV_RANS_OK && r < rounds) {
             // A group of G full rounds takes at most 32 G words and its window
-            // reads 32 ahead, so it cannot run out of words or ring.
-            if (r + G > full || wp + 32 * G + 64 > navail) {
+            // reads 32 ahead, so `groups` of them cannot run out of words.
+            const int64_t spare = (int64_t)navail - (int64_t)wp - 64;
+            int64_t groups = spare > 0 ? spare / (32 * G) : 0;
+            const int64_t left = r < full ? (int64_t)(full - r) / G : 0;
+            if (groups > left) groups = left;
+            if (r == 0 || groups <= 0) {
                 if (!o0_general_round(x, P, r, n, R, wp, navail, out, lt)) status = FQXV_RANS_E_TRUNCATED;
                 r++;
-                window = false;
                 continue;
             }
             R.advance(wp);
             uint32_t w32 = (uint32_t)wp;
-            if (!window) {
-                W = R.at(w32 + lane);
-                e = P[x & (kTotFreq - 1)];
-                window = true;
-            }
+            uint2 W = R.at(w32 + lane);
+            uint32_t e = P[x & (kTotFreq - 1)];
             uint8_t *op = out + r * 32 + lane;
+            r += (uint64_t)groups * G;
+            for (; groups > 0; groups--) {
+                R.follow(w32);
 #pragma unroll
-            for (int g = 0; g < G; g++) {
-                const uint32_t v = ((e >> 20) + 1) * (x >> kScaleBits) + ((e >> 8) & 0xfffu);
-                const uint32_t ev = P[v & (kTotFreq - 1)];
-                const bool need = v < kRansL;
-                const uint32_t mask = __ballot_sync(0xffffffffu, need);
-                const uint32_t srcl = __popc(mask & lt);
-                w32 += __popc(mask);
-                const uint2 nw = R.at(w32 + lane);
-                const uint32_t w = __shfl_sync(0xffffffffu, W.x, srcl);
-                const uint32_t pe = __shfl_sync(0xffffffffu, W.y, srcl);
-                op[32 * g] = (uint8_t)e;
-                x = need ? (v << 16) | w : v;
-                e = need ? pe : ev;
-                W = nw;
+                for (int g = 0; g < G; g++) {
+                    const uint32_t v = ((e >> 20) + 1) * (x >> kScaleBits) + ((e >> 8) & 0xfffu);
+                    const uint32_t ev = P[v & (kTotFreq - 1)];
+                    const bool need = v < kRansL;
+                    const uint32_t mask = __ballot_sync(0xffffffffu, need);
+                    const uint32_t srcl = __popc(mask & lt);
+                    w32 += __popc(mask);
+                    const uint2 nw = R.at(w32 + lane);
+                    const uint32_t w = __shfl_sync(0xffffffffu, W.x, srcl);
+                    const uint32_t pe = __shfl_sync(0xffffffffu, W.y, srcl);
+                    op[32 * g] = (uint8_t)e;
+                    x = need ? __byte_perm(w, v, 0x5410) : v;
+                    e = need ? pe : ev;
+                    W = nw;
+                }
+                op += 32 * G;
             }
             wp += (uint32_t)(w32 - (uint32_t)wp);
-            r += G;
         }
         if (lane == 0) S.status = status;
         __syncwarp();
@@ -923,10 +935,10 @@ __device__ __forceinline__ int o1_rounds(DecStream &S, WordRing<Col> &R, uint8_t
             }
         };
         for (int64_t c = 0; c < cnt; c += kO1Group) {
-            R.advance(wp);
+            R.follow(w32);
             const int m = (int)(cnt - c < kO1Group ? cnt - c : kO1Group);
             if (m == kO1Group && dec.guessing()) {
-                    const uint32_t x0 = x, cb0 = cb, top0 = top;
+                    const uint32_t x0 = x, cb0 = cb, top0 = top, w0 = w32;
                     const D before = dec;
                     bool wrong = false;
 #pragma unroll
@@ -941,7 +953,7 @@ __device__ __forceinline__ int o1_rounds(DecStream &S, WordRing<Col> &R, uint8_t
                         x = x0;
                         cb = cb0;
                         top = top0;
-                        w32 = (uint32_t)wp;
+                        w32 = w0;
                         dec = before;
                         exact_rounds(m);
                     }
@@ -950,8 +962,8 @@ __device__ __forceinline__ int o1_rounds(DecStream &S, WordRing<Col> &R, uint8_t
                 exact_rounds(m);
             }
             op += 32 * m;
-            wp += (uint32_t)(w32 - (uint32_t)wp);
         }
+        wp += (uint32_t)(w32 - (uint32_t)wp);
         r += (uint64_t)cnt;
         if (__any_sync(0xffffffffu, top == kDeadEntry)) status = FQXV_RANS_E_ABSENT_CONTEXT;
     }
