@@ -80,6 +80,7 @@ __global__ void __launch_bounds__(kParseThreads)
             S.ctx0 = 0xff;
             S.cls = kClsNone;
             S.nd = 0;
+            S.nsym = 0;
             S.start = 0;
             S.tbl_bytes = 0;
         }
@@ -191,19 +192,31 @@ __global__ void __launch_bounds__(kParseThreads)
             if (status == FQXV_RANS_OK && L < hdr + kStatesBytes) status = FQXV_RANS_E_TRUNCATED;
             if (status == FQXV_RANS_OK && n > S.dst_cap) status = FQXV_RANS_E_ALLOC;
             if (status == FQXV_RANS_OK) {
-                // D = present contexts plus every symbol of their tables.
+                // D = every symbol of the present contexts' tables, in byte
+                // order, then the present contexts that are no symbol (as a
+                // rule context 0 alone, which only the first position has):
+                // the decoders' contexts are then the first S.nsym indices.
                 if (warp == 0) {
-                    uint32_t flags = 0;
+                    uint32_t syms = 0, others = 0;
 #pragma unroll
                     for (int k = 0; k < 8; k++) {
                         const int s = lane * 8 + k;
-                        if (symseen[s] || ctxmap[s] != 0xff) flags |= 1u << k;
+                        if (symseen[s]) syms |= 1u << k;
+                        else if (ctxmap[s] != 0xff) others |= 1u << k;
                     }
-                    const uint32_t c = __popc(flags);
-                    uint32_t base = warp_incl_scan(c) - c;
+                    const uint32_t c = __popc(syms), o = __popc(others);
+                    const uint32_t ci = warp_incl_scan(c), oi = warp_incl_scan(o);
+                    const uint32_t ns = __shfl_sync(0xffffffffu, ci, 31);
+                    uint32_t base = ci - c, obase = ns + oi - o;
 #pragma unroll
-                    for (int k = 0; k < 8; k++) dmap[lane * 8 + k] = (flags >> k) & 1u ? (uint8_t)(base++) : 0xff;
-                    if (lane == 31) s_nd = (int)base;
+                    for (int k = 0; k < 8; k++)
+                        dmap[lane * 8 + k] = (syms >> k) & 1u     ? (uint8_t)(base++)
+                                             : (others >> k) & 1u ? (uint8_t)(obase++)
+                                                                  : 0xff;
+                    if (lane == 31) {
+                        s_nd = (int)(ns + oi);
+                        S.nsym = (int)ns;
+                    }
                 }
                 __syncthreads();
                 const int nd = s_nd;
@@ -1006,14 +1019,16 @@ struct DenseImage {
 // and composing is a shuffle (h[c] = g[f[c]]), three levels for eight columns.
 // When the context arrives, three shuffles give all eight symbols, and the
 // context goes on to the next warp at once. With contexts of 32 and up (HI,
-// |D| > 32) a function takes two registers and a composition four shuffles;
+// more than 32 symbols) a function takes two registers and a composition four shuffles;
 // there each lane walks columns 0-3 and 4-7 from contexts lane and lane + 32
 // by byte loads, and only the second walk is composed after the first.
 //
 // What bounds it is a warp's own loop, about 130 instructions, most of them
 // in one dependent chain (a hop to the next warp is ~85 cycles, four a round
-// ~340). One stream, cycles per round: full-range quality (|D| = 31) 529, ONT
-// quality (39) 601, random walk (41) 598. Before, every warp held all 32
+// ~340). One stream, cycles per round: full-range quality (31 or 32 symbols)
+// 529, ONT quality (39) 601, random walk (41) 598; a context 0 that is no
+// symbol once counted, and took the streams of 32 symbols to the wider form's
+// 601. Before, every warp held all 32
 // states, ran a segment's chains from every context and followed three rows
 // of shared memory behind a barrier: 642, 614 and 615.
 constexpr int kO1Warps = 4;
@@ -1287,8 +1302,9 @@ __global__ void __launch_bounds__(kO1Threads, 4)
         R.init(src + S.words_off, S.words_len, sm + ring_off + warp * kRingBytes);
         uint8_t *out = dst + S.dst_off;
         // 32 symbols leave no lane for DEAD, and need none: a stream that meets
-        // it has failed, and any context may follow.
-        const int status = S.nd <= 32 ? relay_stream<false>(sh, S, I, R, out, lt)
+        // it has failed, and any context may follow. A context that is no
+        // symbol is the first position's, which is not among these rounds.
+        const int status = S.nsym <= 32 ? relay_stream<false>(sh, S, I, R, out, lt)
                                       : relay_stream<true>(sh, S, I, R, out, lt);
         if (tid == 0) s_status = S.status = status;
         __syncthreads();

@@ -85,6 +85,7 @@ struct DecStream {
     int32_t ctx0;                // global format: dense index of context 0 (0xFF: absent)
     int32_t cls;                 // decode class (kClsO0, kClsO1Dense, kClsO1Global)
     int32_t nd;                  // dense format: |D| (symbols and contexts), DEAD = nd
+    int32_t nsym;                // dense format: symbols, the first indices of D
     int32_t start;               // dense format: index of context 0 (DEAD when absent)
     uint32_t tbl_bytes;          // bytes of the table image staged into shared memory
     uint32_t states[kStates];
@@ -107,12 +108,13 @@ constexpr int kMidMaxNd = 15;
 // Decode table arena per stream (bytes from tbl_off).
 //   order-0: 4096 x u32 packed ((freq - 1) << 20) | ((slot - cum) << 8) | sym.
 //   order-1 dense (|D| <= kDenseMax and an image of at most kDenseImageMax
-//     bytes): D = present contexts and every symbol of their tables, in
-//     ascending byte order; DEAD = |D| marks "absent context". The slot axis
-//     is cut at every position where some context's symbol changes (a
-//     boundary: a cum value of a present symbol); between two boundaries
-//     every context decodes every slot to the same symbol, so one column per
-//     boundary holds, for each context, the dense symbol of that slot range.
+//     bytes): D = every symbol of the present contexts' tables, then the
+//     present contexts that are no symbol, each in byte order; DEAD = |D|
+//     marks "absent context". The slot axis is cut at every position where
+//     some context's symbol changes (a boundary: a cum value of a present
+//     symbol); between two boundaries every context decodes every slot to the
+//     same symbol, so one column per boundary holds, for each context, the
+//     dense symbol of that slot range.
 //     [0, 4096)                 M8: u8 per slot, the slot's column less the
 //                               first column of its 256-slot block
 //     [4096, 4160)              MB: u32 per 256-slot block, that first

@@ -75,3 +75,49 @@ def test_guessed_contexts_match_oracle(orc, nsym, make):
     finally:
         codec.close()
     assert rans.decode(streams[-1]) == blocks[-1].tobytes()
+
+
+@pytest.mark.parametrize("nsym", [31, 32, 33])
+@pytest.mark.parametrize("zero", [False, True])
+def test_first_context_need_not_be_a_symbol(orc, nsym, zero):
+    """Context 0 takes an index behind the symbols' when byte 0 never occurs:
+    around the 32 lanes of the four-warp decoder, good streams and streams with
+    damaged words (which meet symbols that have no context) decode as the
+    oracle's do."""
+    import torch
+
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from fqxv_b200.batch import Codec
+
+    rng = np.random.default_rng(100 * nsym + zero)
+    alphabet = _symbols(rng, nsym)
+    if zero:
+        alphabet[0] = 0
+    streams = []
+    for i, n in enumerate([1, 33, 5 * GROUP + 9, 40_001, 60_000, 60_000]):
+        block = _iid(rng, alphabet[:-1], n)
+        block[-1] = alphabet[-1]  # the last symbol has no context of its own
+        s = bytearray(orc.encode(block.tobytes(), 1))
+        if i >= 4:
+            s[len(s) * 3 // 4] ^= 0x55
+        streams.append(bytes(s))
+    want = [orc.decode_status(s, max_len=1 << 16) for s in streams]
+    lens = np.array([len(s) for s in streams], np.uint64)
+    offs = np.concatenate([[0], np.cumsum(lens)[:-1]]).astype(np.uint64)
+    out_offs = np.arange(len(streams), dtype=np.uint64) << np.uint64(16)
+    out_spans = np.stack([out_offs, np.full(len(streams), 1 << 16, np.uint64)], axis=1)
+    d_src = torch.from_numpy(np.frombuffer(b"".join(streams), np.uint8).copy()).to("cuda")
+    codec = Codec(0)
+    try:
+        for top_max in (0, 1000):
+            codec.set_param("o1_top_max", top_max)
+            out, got, status = codec.decode_batch(d_src, np.stack([offs, lens], 1), out_spans, max_len=1 << 16,
+                                                  raise_on_error=False)
+            out = out.cpu().numpy()
+            for i, (ws, wb) in enumerate(want):
+                assert status[i] == ws, (top_max, i)
+                if ws == 0:
+                    assert out[int(out_offs[i]):int(out_offs[i]) + int(got[i])].tobytes() == wb, (top_max, i)
+    finally:
+        codec.close()
