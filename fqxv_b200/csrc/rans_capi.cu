@@ -324,20 +324,45 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
             const double lat = (double)d.n * lat_cpb(d);
             if (d.cls == kClsO1Dense && lat > top_thr) cand.emplace_back(lat, (uint32_t)i);
         }
-        const size_t ntop = std::min<size_t>(cand.size(), (size_t)std::max<int64_t>(top_max, 0));
-        std::partial_sort(cand.begin(), cand.begin() + ntop, cand.end(),
+        size_t ntop = std::min<size_t>(cand.size(), (size_t)std::max<int64_t>(top_max, 0));
+        std::partial_sort(cand.begin(), cand.begin() + std::min(ntop + 1, cand.size()), cand.end(),
                           [](const std::pair<double, uint32_t> &a, const std::pair<double, uint32_t> &b) {
                               return a.first > b.first || (a.first == b.first && a.second < b.second);
                           });
+        // Like-sized streams have no such longest ones: those left out, on the
+        // SMs that remain, would finish last instead (600 full-range blocks of
+        // 256 KiB: 7.7 ms with top groups, 4.3 without; mixed batches of 2048
+        // and 4096 blocks, whose first left out take 0.5 to 0.7 of the longest:
+        // 35 and 47 ms, 62 and 65 without).
+        if (ntop && ntop < cand.size() && cand[ntop].first > 0.8 * cand[0].first) ntop = 0;
         std::vector<uint8_t> is_top(nb, 0);
         for (size_t k = 0; k < ntop; k++) is_top[cand[k].second] = 1;
+        // Small-alphabet top streams share an SM, top_pack to one, where each
+        // takes a tenth longer than alone (names of 1 MiB: 9.4 ms or 8.5).
+        // Those that would outlast every other stream by that get an SM each,
+        // longest first, while the other top streams and the rest (its SM
+        // cycles over the longest stream's time) leave SMs for it.
+        const int64_t top_pack = ctx->tune.o1_top_small_per_sm;
+        if (ntop && top_pack > 1) {
+            double rest = 0;
+            int64_t four = 0, packed = 0;
+            for (size_t i = 0; i < nb; i++)
+                if (is_top[i]) (ps[i].nd > kMidMaxNd ? four : packed)++;
+                else if (ps[i].cls != kClsNone) rest += (double)ps[i].n * rate_cpb(ps[i]);
+            double spare = (double)(ctx->sms - four) - rest / cand[0].first - (double)packed / (double)top_pack;
+            for (size_t k = 0; k < ntop && spare >= 1.0 && cand[k].first * 1.15 > cand[0].first; k++) {
+                if (ps[cand[k].second].nd > kMidMaxNd) continue;
+                is_top[cand[k].second] = 2;
+                spare -= 1.0 - 1.0 / (double)top_pack;
+            }
+        }
         auto group_of = [&](uint32_t i) -> int {
             const DecStream &d = ps[i];
             if (d.cls == kClsO0) return 0;
             if (d.cls == kClsO1Global) return kGroups - 1;
             if (d.cls != kClsO1Dense) return -1;
-            if (d.nd <= kTinyMaxNd) return is_top[i] ? kGroupTinyTop : kGroupTiny;
-            if (d.nd <= kMidMaxNd) return is_top[i] ? kGroupMidTop : kGroupMid;
+            if (d.nd <= kTinyMaxNd) return is_top[i] == 2 ? kGroupTinyAlone : is_top[i] ? kGroupTinyTop : kGroupTiny;
+            if (d.nd <= kMidMaxNd) return is_top[i] == 2 ? kGroupMidAlone : is_top[i] ? kGroupMidTop : kGroupMid;
             if (is_top[i]) return kGroupFourTop;
             return d.tbl_bytes <= (uint64_t)ctx->tune.dense_edge_small   ? kGroupDense0
                    : d.tbl_bytes <= (uint64_t)ctx->tune.dense_edge_large ? kGroupDense0 + 1
@@ -357,22 +382,28 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
             maxlat[g] = std::max(maxlat[g], (double)ps[i].n * lat_cpb(ps[i]));
             ndmax[g] = std::max(ndmax[g], ps[i].nd);
         }
-        int gcls[kGroups];
+        int gcls[kGroups], top_warps[kGroups] = {};
         uint32_t smem[kGroups];
-        const int64_t four_max = ctx->tune.o1_four_max_streams < 0 ? ctx->sms : ctx->tune.o1_four_max_streams;
+        const int64_t four_max = ctx->tune.o1_four_max_streams < 0 ? 3 * ctx->sms : ctx->tune.o1_four_max_streams;
         for (int g = 0; g < kGroups; g++) {
             if (g == 0) gcls[g] = kClsO0;
             else if (g == kGroups - 1) gcls[g] = kClsO1Global;
-            else if (g == kGroupTiny || g == kGroupTinyTop) gcls[g] = kClsO1Small;
-            else if (g == kGroupMid || g == kGroupMidTop) gcls[g] = kClsO1Mid;
+            else if (g == kGroupTiny || g == kGroupTinyTop || g == kGroupTinyAlone) gcls[g] = kClsO1Small;
+            else if (g == kGroupMid || g == kGroupMidTop || g == kGroupMidAlone) gcls[g] = kClsO1Mid;
             else if (g == kGroupFourTop) gcls[g] = kClsO1Dense;
-            else gcls[g] = (int64_t)lists[g].size() < four_max ? kClsO1Dense : kClsO1Wide;
+            else gcls[g] = (int64_t)nb <= four_max ? kClsO1Dense : kClsO1Wide;
             smem[g] = dec_smem_bytes(gcls[g], tmax[g], ndmax[g]);
-            // the groups of largest streams: one CTA per SM, alone on it
-            if (is_top_group(g) && ctx->tune.o1_top_exclusive)
-                smem[g] = std::max(smem[g], dec_exclusive_smem(gcls[g], g == kGroupFourTop
-                                                                              ? 1
-                                                                              : (int)ctx->tune.o1_top_small_per_sm));
+            // The groups of largest streams: one CTA per SM, alone on it. One
+            // of small alphabets takes up to top_pack streams, as far as
+            // their tables fit.
+            if (is_top_group(g) && ctx->tune.o1_top_exclusive) {
+                if (g == kGroupTinyTop || g == kGroupMidTop) {
+                    const uint32_t all = dec_exclusive_smem(gcls[g], true);
+                    top_warps[g] = (int)std::min<int64_t>(top_pack, all / smem[g]);
+                    if (top_warps[g] < 2) top_warps[g] = 0;
+                }
+                smem[g] = std::max(smem[g], dec_exclusive_smem(gcls[g], top_warps[g] != 0));
+            }
         }
         // Groups are launched longest first -- by the serial time of their
         // largest stream (lat_cpb above) -- so the streams that bound the batch take SMs
@@ -405,7 +436,7 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
                                                                                          : kStDecO1Dense;
             cudaStream_t as = ctx->aux[g];
             CK(cudaStreamWaitEvent(as, ctx->ev_fork, 0));
-            int per_sm = dec_blocks_per_sm(cls, smem[g]);
+            int per_sm = top_warps[g] ? 1 : dec_blocks_per_sm(cls, smem[g]);
             const Tuning &T = ctx->tune;
             const bool small = cls == kClsO1Small || cls == kClsO1Mid;
             int64_t cap = cls == kClsO0 ? T.cta_cap_o0 : small ? T.cta_cap_o1_small
@@ -420,16 +451,17 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
             per_sm = std::max(1, std::min<int>(per_sm, (int)cap));
             ctx->timer.shape(stage, per_sm, smem[g]);
             if (persistent) {
-                const int grid = (int)std::min<size_t>(m, (size_t)ctx->sms * per_sm);
+                const size_t at_once = (size_t)std::max(top_warps[g], 1);
+                const int grid = (int)std::min<size_t>((m + at_once - 1) / at_once, (size_t)ctx->sms * per_sm);
                 cudaEvent_t t0 = ctx->timer.begin(as);
-                launch_dec_run(cls, d_src, dS, dl + base[g], (int)m, dT, d_dst, queue + 4 * g, grid, smem[g],
+                launch_dec_run(cls, d_src, dS, dl + base[g], (int)m, dT, d_dst, queue + 4 * g, grid, top_warps[g], smem[g],
                                ctx->first_polls, mirror, as);
                 ctx->timer.end(stage, t0, as);
             } else {
                 for (size_t j = 0; j < m; j++) {
                     CK(cudaMemsetAsync(queue + 4 * g, 0, 4, as));
                     cudaEvent_t t0 = ctx->timer.begin(as);
-                    launch_dec_run(cls, d_src, dS, dl + base[g] + j, 1, dT, d_dst, queue + 4 * g, 1,
+                    launch_dec_run(cls, d_src, dS, dl + base[g] + j, 1, dT, d_dst, queue + 4 * g, 1, 0,
                                    dec_smem_bytes(cls, ps[lists[g][j]].tbl_bytes, ps[lists[g][j]].nd),
                                    ctx->first_polls, mirror, as);
                     ctx->timer.end(stage, t0, as);

@@ -77,7 +77,8 @@ struct HostBuf {
 // up to kMidMaxNd symbols; order-1 wide alphabets in three table-size ranges;
 // the order-1 streams that bound the batch by their serial time, wide
 // alphabets (four-warp decoder), tiny ones and those between, each group on
-// SMs of its own; order-1 global tables.
+// SMs of its own, and of the latter two the streams that take an SM each;
+// order-1 global tables.
 constexpr int kGroupTiny = 1;
 constexpr int kGroupMid = 2;
 constexpr int kGroupDense0 = 3;   // first of the three dense table-size groups
@@ -85,8 +86,10 @@ constexpr int kDenseGroups = 3;
 constexpr int kGroupFourTop = kGroupDense0 + kDenseGroups;
 constexpr int kGroupTinyTop = kGroupFourTop + 1;
 constexpr int kGroupMidTop = kGroupTinyTop + 1;
-constexpr int kGroups = kGroupMidTop + 2;
-inline bool is_top_group(int g) { return g >= kGroupFourTop && g <= kGroupMidTop; }
+constexpr int kGroupTinyAlone = kGroupMidTop + 1;
+constexpr int kGroupMidAlone = kGroupTinyAlone + 1;
+constexpr int kGroups = kGroupMidAlone + 2;
+inline bool is_top_group(int g) { return g >= kGroupFourTop && g <= kGroupMidAlone; }
 
 enum Stage {
     kStEncModel, kStEncRun, kStEncScan, kStEncPack, kStDecParse, kStDecO0, kStDecO1Dense, kStDecO1Global,
@@ -102,23 +105,26 @@ const char *const kStageNames[kStages] = {"enc_model", "enc_run", "enc_select_sc
 // them.
 struct Tuning {
     // Order-1 streams of more than kMidMaxNd symbols with shared-memory
-    // tables: a launch group of fewer than this many goes to the four-warp
-    // decoder (one stream per SM), larger groups to the one-warp decoder
-    // (several per SM). -1: the SM count.
+    // tables: batches of at most this many streams send them to the four-warp
+    // decoder, larger ones (the top group aside) to the one-warp decoder. -1:
+    // three to an SM (full-range blocks of 256 KiB, four-warp and one-warp:
+    // 200 of them 2.65 and 3.88 ms, 444 of them 3.48 and 3.95, 592 4.4 and 4.3).
     int64_t o1_four_max_streams = -1;
     // Order-1 streams whose serial decode alone outlasts o1_top_latency_pct %
     // of the batch's throughput-bound time -- the o1_top_max longest of them
     // -- form launch groups of their own (the batch lasts at least as long as
     // its longest serial chain): wide alphabets on the four-warp decoder,
     // small ones on the one-warp decoder. o1_top_max -1: half the SM count.
+    // None when the longest left out is nearly as long.
     int64_t o1_top_latency_pct = 75;
     int64_t o1_top_max = -1;
     // 1: those two groups run one CTA per SM with no other CTA beside it
     // (their CTAs claim the SM's shared memory), so their serial chains are
     // not slowed by the rest of the batch; 0: they share.
     int64_t o1_top_exclusive = 1;
-    // CTAs per SM of the small-alphabet top group when exclusive: each is one
-    // warp, so up to four can hold an SM together, one per scheduler.
+    // Streams per SM of the small-alphabet top groups when exclusive: the
+    // warps of one CTA, so up to four hold an SM together, one per scheduler;
+    // the longest of them take an SM each.
     int64_t o1_top_small_per_sm = 4;
     // CTAs per SM of each decode class, at most (the occupancy API bounds it too)
     int64_t cta_cap_o0 = 32, cta_cap_o1_small = 32, cta_cap_o1_wide = 32, cta_cap_o1_four = 8,

@@ -1607,21 +1607,29 @@ __device__ __forceinline__ int o1w_stream(DecStream &S, const uint8_t *__restric
 // kernel to 96 registers and puts the column loads one behind the other
 // (full-range quality, one stream: 1430 cycles a round at 96 registers, 850
 // at 152).
-template <int kCls>
-__global__ void __launch_bounds__(32, kCls == kClsO1Wide ? 8 : 16)
+// kWarps > 1: up to that many streams in a CTA, a warp and a slice of the
+// dynamic shared memory each, for the top groups: as CTAs of their own they
+// are dealt out one to an SM, and each shares it with the rest of the batch
+// (4 MiB of names among 2048 mixed blocks: 39 ms, alone 33, four alone on an
+// SM 35).
+template <int kCls, int kWarps>
+__global__ void __launch_bounds__(32 * kWarps, (kCls == kClsO1Wide ? 8 : 16) / kWarps)
     dec_o1w_kernel(const uint8_t *__restrict__ src, DecStream *__restrict__ streams,
                    const uint32_t *__restrict__ list, int nlist, const uint8_t *__restrict__ tbl,
-                   uint8_t *__restrict__ dst, int *__restrict__ queue, uint32_t ring_off,
+                   uint8_t *__restrict__ dst, int *__restrict__ queue, uint32_t slice, uint32_t ring_off,
                    uint32_t first_polls, uint8_t *__restrict__ mirror) {
-    extern __shared__ __align__(128) uint8_t sm[];
-    __shared__ __align__(8) uint64_t bar;
-    __shared__ __align__(16) uint8_t s_xch[kCls == kClsO1Small ? TinyDecoder::kBytes
-                                           : kCls == kClsO1Mid ? MidDecoder::kBytes
-                                                               : WideDecoder<2>::kBytes];
-    const int lane = threadIdx.x;
+    extern __shared__ __align__(128) uint8_t smem[];
+    constexpr int kXch = kCls == kClsO1Small ? TinyDecoder::kBytes
+                         : kCls == kClsO1Mid ? MidDecoder::kBytes
+                                             : WideDecoder<2>::kBytes;
+    __shared__ __align__(8) uint64_t bars[kWarps];
+    __shared__ __align__(16) uint8_t s_xchs[kWarps][kXch];
+    const int warp = kWarps > 1 ? threadIdx.x >> 5 : 0, lane = threadIdx.x & 31;
+    uint8_t *sm = smem + warp * slice;
+    uint8_t *s_xch = s_xchs[warp];
     const uint32_t lt = lanemask_lt();
     TableStager st;
-    st.init(&bar);
+    st.init(&bars[warp]);
     bool stuck = false;
     for (;;) {
         const int j = pop_job(queue);
@@ -1767,29 +1775,29 @@ uint32_t dec_smem_bytes(int cls, uint32_t tbl_bytes, int nd) {
 
 // Dynamic shared memory of one CTA that leaves no room on its SM for any
 // other: the per-block opt-in maximum less the kernel's static shared memory.
-// With per_sm > 1: the share that lets exactly per_sm such CTAs fill an SM
-// (each CTA also costs its static shared memory and the 1 KB the driver
-// reserves per block).
-static uint32_t exclusive_bytes(const void *fn, int per_sm) {
-    int dev = 0, optin = 0, per_smem = 0;
+static uint32_t exclusive_bytes(const void *fn) {
+    int dev = 0, optin = 0;
     cudaFuncAttributes a;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&per_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
         cudaFuncGetAttributes(&a, fn) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
-    int64_t b = (int64_t)optin - (int64_t)a.sharedSizeBytes;
-    if (per_sm > 1) b = std::min<int64_t>(b, (int64_t)per_smem / per_sm - 1024 - (int64_t)a.sharedSizeBytes);
+    const int64_t b = (int64_t)optin - (int64_t)a.sharedSizeBytes;
     return b > 0 ? (uint32_t)b / 128 * 128 : 0u;
 }
 
-uint32_t dec_exclusive_smem(int cls, int per_sm) {
-    if (cls == kClsO1Dense) return exclusive_bytes(reinterpret_cast<const void *>(dec_o1d_kernel), per_sm);
-    if (cls == kClsO1Small) return exclusive_bytes(reinterpret_cast<const void *>(dec_o1w_kernel<kClsO1Small>), per_sm);
-    if (cls == kClsO1Mid) return exclusive_bytes(reinterpret_cast<const void *>(dec_o1w_kernel<kClsO1Mid>), per_sm);
-    return 0;
+uint32_t dec_exclusive_smem(int cls, bool top) {
+    const void *fn = nullptr;
+    if (cls == kClsO1Dense) fn = reinterpret_cast<const void *>(dec_o1d_kernel);
+    if (cls == kClsO1Small)
+        fn = top ? reinterpret_cast<const void *>(dec_o1w_kernel<kClsO1Small, kO1TopWarps>)
+                 : reinterpret_cast<const void *>(dec_o1w_kernel<kClsO1Small, 1>);
+    if (cls == kClsO1Mid)
+        fn = top ? reinterpret_cast<const void *>(dec_o1w_kernel<kClsO1Mid, kO1TopWarps>)
+                 : reinterpret_cast<const void *>(dec_o1w_kernel<kClsO1Mid, 1>);
+    return fn ? exclusive_bytes(fn) : 0;
 }
 
 // Each decode kernel's dynamic shared-memory limit is raised once per
@@ -1813,22 +1821,30 @@ static void ensure_dec_attrs() {
                          (int)std::max(dec_smem_bytes(kClsO1Dense, kDenseImageMax), dec_exclusive_smem(kClsO1Dense)));
     cudaFuncSetAttribute(dec_o1g_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)dec_smem_bytes(kClsO1Global, 0));
-    cudaFuncSetAttribute(dec_o1w_kernel<kClsO1Small>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(dec_o1w_kernel<kClsO1Small, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)std::max(dec_smem_bytes(kClsO1Small, kTinyBytes), dec_exclusive_smem(kClsO1Small)));
-    cudaFuncSetAttribute(dec_o1w_kernel<kClsO1Wide>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)dec_smem_bytes(kClsO1Wide, kDenseImageMax));
-    cudaFuncSetAttribute(dec_o1w_kernel<kClsO1Mid>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(dec_o1w_kernel<kClsO1Mid, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)std::max(dec_smem_bytes(kClsO1Mid, kDenseImageMax), dec_exclusive_smem(kClsO1Mid)));
+    cudaFuncSetAttribute(dec_o1w_kernel<kClsO1Wide, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)dec_smem_bytes(kClsO1Wide, kDenseImageMax));
+    cudaFuncSetAttribute(dec_o1w_kernel<kClsO1Small, kO1TopWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)dec_exclusive_smem(kClsO1Small, true));
+    cudaFuncSetAttribute(dec_o1w_kernel<kClsO1Mid, kO1TopWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)dec_exclusive_smem(kClsO1Mid, true));
     // Kernels whose tables live in shared memory take the largest shared-
     // memory share of the SM's L1, so as many streams as fit run per SM (the
     // global-table decoder keeps its L1 for the tables it reads through it).
     cudaFuncSetAttribute(dec_o0_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     cudaFuncSetAttribute(dec_o1d_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    cudaFuncSetAttribute(dec_o1w_kernel<kClsO1Small>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    cudaFuncSetAttribute(dec_o1w_kernel<kClsO1Small, 1>, cudaFuncAttributePreferredSharedMemoryCarveout,
                          cudaSharedmemCarveoutMaxShared);
-    cudaFuncSetAttribute(dec_o1w_kernel<kClsO1Wide>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    cudaFuncSetAttribute(dec_o1w_kernel<kClsO1Mid, 1>, cudaFuncAttributePreferredSharedMemoryCarveout,
                          cudaSharedmemCarveoutMaxShared);
-    cudaFuncSetAttribute(dec_o1w_kernel<kClsO1Mid>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    cudaFuncSetAttribute(dec_o1w_kernel<kClsO1Wide, 1>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                         cudaSharedmemCarveoutMaxShared);
+    cudaFuncSetAttribute(dec_o1w_kernel<kClsO1Small, kO1TopWarps>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                         cudaSharedmemCarveoutMaxShared);
+    cudaFuncSetAttribute(dec_o1w_kernel<kClsO1Mid, kO1TopWarps>, cudaFuncAttributePreferredSharedMemoryCarveout,
                          cudaSharedmemCarveoutMaxShared);
     cudaGetLastError();
     g_attr_done[dev] = true;
@@ -1849,13 +1865,13 @@ int dec_blocks_per_sm(int cls, uint32_t smem_bytes) {
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dec_o1g_kernel, 32, smem_bytes);
             break;
         case kClsO1Small:
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dec_o1w_kernel<kClsO1Small>, 32, smem_bytes);
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dec_o1w_kernel<kClsO1Small, 1>, 32, smem_bytes);
             break;
         case kClsO1Mid:
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dec_o1w_kernel<kClsO1Mid>, 32, smem_bytes);
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dec_o1w_kernel<kClsO1Mid, 1>, 32, smem_bytes);
             break;
         case kClsO1Wide:
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dec_o1w_kernel<kClsO1Wide>, 32, smem_bytes);
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, dec_o1w_kernel<kClsO1Wide, 1>, 32, smem_bytes);
             break;
         default:
             break;
@@ -1874,9 +1890,11 @@ void launch_dec_parse(const uint8_t *src, DecStream *streams, int nstreams, uint
 }
 
 void launch_dec_run(int cls, const uint8_t *src, DecStream *streams, const uint32_t *list, int nlist,
-                    const uint8_t *tbl, uint8_t *dst, int *queue, int grid, uint32_t smem_bytes,
+                    const uint8_t *tbl, uint8_t *dst, int *queue, int grid, int top_warps, uint32_t smem_bytes,
                     uint32_t first_polls, uint8_t *mirror, cudaStream_t s) {
     if (nlist <= 0 || grid <= 0) return;
+    // each warp's share, whole 128-byte lines
+    const uint32_t slice = smem_bytes / (uint32_t)std::max(top_warps, 1) / 128 * 128;
     ensure_dec_attrs();
     switch (cls) {
         case kClsO0:
@@ -1891,17 +1909,29 @@ void launch_dec_run(int cls, const uint8_t *src, DecStream *streams, const uint3
         case kClsO1Global:
             dec_o1g_kernel<<<grid, 32, smem_bytes, s>>>(src, streams, list, nlist, tbl, dst, queue, mirror);
             break;
-        case kClsO1Small:
-            dec_o1w_kernel<kClsO1Small><<<grid, 32, smem_bytes, s>>>(src, streams, list, nlist, tbl, dst, queue,
-                                                                smem_bytes - 2 * kRingBytes, first_polls, mirror);
+        case kClsO1Small: {
+            const uint32_t ring = slice - 2 * kRingBytes;
+            if (top_warps)
+                dec_o1w_kernel<kClsO1Small, kO1TopWarps><<<grid, 32 * top_warps, smem_bytes, s>>>(
+                    src, streams, list, nlist, tbl, dst, queue, slice, ring, first_polls, mirror);
+            else
+                dec_o1w_kernel<kClsO1Small, 1><<<grid, 32, smem_bytes, s>>>(src, streams, list, nlist, tbl, dst, queue,
+                                                                            slice, ring, first_polls, mirror);
             break;
-        case kClsO1Mid:
-            dec_o1w_kernel<kClsO1Mid><<<grid, 32, smem_bytes, s>>>(src, streams, list, nlist, tbl, dst, queue,
-                                                                   smem_bytes - kRingBytes, first_polls, mirror);
+        }
+        case kClsO1Mid: {
+            const uint32_t ring = slice - kRingBytes;
+            if (top_warps)
+                dec_o1w_kernel<kClsO1Mid, kO1TopWarps><<<grid, 32 * top_warps, smem_bytes, s>>>(
+                    src, streams, list, nlist, tbl, dst, queue, slice, ring, first_polls, mirror);
+            else
+                dec_o1w_kernel<kClsO1Mid, 1><<<grid, 32, smem_bytes, s>>>(src, streams, list, nlist, tbl, dst, queue,
+                                                                          slice, ring, first_polls, mirror);
             break;
+        }
         case kClsO1Wide:
-            dec_o1w_kernel<kClsO1Wide><<<grid, 32, smem_bytes, s>>>(src, streams, list, nlist, tbl, dst, queue,
-                                                               smem_bytes - kRingBytes, first_polls, mirror);
+            dec_o1w_kernel<kClsO1Wide, 1><<<grid, 32, smem_bytes, s>>>(src, streams, list, nlist, tbl, dst, queue, slice,
+                                                                       slice - kRingBytes, first_polls, mirror);
             break;
         default:
             break;

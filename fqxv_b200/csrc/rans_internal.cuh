@@ -104,6 +104,9 @@ constexpr int kClsO1Mid = 6;
 constexpr int kTinyMaxNd = 5;
 // 16 entries of a byte column fit in four registers.
 constexpr int kMidMaxNd = 15;
+// Warps of an exclusive top group's CTA of those two classes, at most: one
+// per scheduler.
+constexpr int kO1TopWarps = 4;
 
 // Decode table arena per stream (bytes from tbl_off).
 //   order-0: 4096 x u32 packed ((freq - 1) << 20) | ((slot - cum) << 8) | sym.
@@ -203,9 +206,11 @@ void launch_dec_parse(const uint8_t *src, DecStream *streams, int nstreams, uint
 // smem_bytes is the dynamic shared memory of the class (largest member).
 // `mirror` (nullable): each stream decoded without error is also copied to
 // mirror + dst_off (the device alias of a pinned host destination) by the
-// CTA that decoded it.
+// CTA that decoded it. top_warps (kClsO1Small and kClsO1Mid): 0, or the
+// streams each CTA decodes at a time, a warp and an equal share of smem_bytes
+// each (an exclusive top group's launch).
 void launch_dec_run(int cls, const uint8_t *src, DecStream *streams, const uint32_t *list, int nlist,
-                    const uint8_t *tbl, uint8_t *dst, int *queue, int grid, uint32_t smem_bytes,
+                    const uint8_t *tbl, uint8_t *dst, int *queue, int grid, int top_warps, uint32_t smem_bytes,
                     uint32_t first_polls, uint8_t *mirror, cudaStream_t s);
 // `nd`: the largest |D| among the launch's streams (the one-warp wide
 // decoder keeps its rows, 3 |D| + 2 per buffer, in dynamic shared memory).
@@ -213,9 +218,9 @@ uint32_t dec_smem_bytes(int cls, uint32_t tbl_bytes, int nd = kDenseMax);
 // Bytes of the one-warp wide decoder's two row buffers for |D| = nd.
 __host__ __device__ inline uint32_t wide_rows_bytes(int nd) { return (uint32_t)((2 * (3 * nd + 2) * 16 + 127) / 128 * 128); }
 // Dynamic shared memory with which one CTA of a decode class fills an SM (no
-// other CTA fits beside it); 0 when the class cannot.
-// per_sm > 1: the share that lets exactly per_sm such CTAs fill an SM.
-uint32_t dec_exclusive_smem(int cls, int per_sm = 1);
+// other CTA fits beside it); 0 when the class cannot. `top`: of the kernel
+// that decodes several streams per CTA.
+uint32_t dec_exclusive_smem(int cls, bool top = false);
 // CTAs of a decode class that fit on one SM with `smem_bytes` of dynamic
 // shared memory (registers and static shared memory included).
 int dec_blocks_per_sm(int cls, uint32_t smem_bytes);

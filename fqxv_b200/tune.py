@@ -17,13 +17,14 @@ reference's only run-time choice is its SIMD backend
   o1_top_max            at most this many streams (the longest) in those
                         groups
   o1_top_exclusive      1: those two groups run on SMs of their own
-  o1_top_small_per_sm   CTAs (one warp each) per such SM of the small group
+  o1_top_small_per_sm   streams (a warp each of one CTA) per such SM of the
+                        small group; its longest take an SM each
   enc_o1_keys           order-1 encode reads per-position table indices stored
                         by the model kernel (1) or derives them (0)
-  o1_four_max_streams   below this many wide-alphabet order-1 streams in a
-                        launch group the four-warp decoder (one stream per
-                        SM, lower latency per stream) runs them, else the
-                        one-warp decoder (several streams per SM)
+  o1_four_max_streams   batches of at most this many streams send wide-
+                        alphabet order-1 streams to the four-warp decoder
+                        (lower latency per stream), larger ones to the
+                        one-warp decoder (more streams per SM)
   cta_cap_o1_small_topped / cta_cap_o1_wide_topped
                         the same outside the top groups of a batch that has
                         them (its largest bulk streams run less contended)
@@ -165,7 +166,7 @@ def sweep(reps: int = 3) -> dict:
     pick("o1_top_latency_pct", (25, 50, 75, 100, 150, 100000), score)
     pick("o1_top_max", (sms // 4, sms // 2, 3 * sms // 4, sms), score)
     pick("o1_top_small_per_sm", (1, 2, 4), score)
-    pick("o1_four_max_streams", (0, sms // 2, sms, 2 * sms, 4 * sms, 1 << 30), score)
+    pick("o1_four_max_streams", (0, sms // 2, sms, 2 * sms, 3 * sms, 4 * sms, 1 << 30), score)
     # one-warp CTAs per SM outside the top groups, when a batch has them
     pick("cta_cap_o1_small_topped", (2, 4, 8, 16), lambda: bm.decode_gbs(reps))
     pick("cta_cap_o1_wide_topped", (2, 3, 4, 6), lambda: bm.decode_gbs(reps))

@@ -121,3 +121,37 @@ def test_first_context_need_not_be_a_symbol(orc, nsym, zero):
                     assert out[int(out_offs[i]):int(out_offs[i]) + int(got[i])].tobytes() == wb, (top_max, i)
     finally:
         codec.close()
+
+
+@pytest.mark.parametrize("per_sm", [1, 2, 3, 4])
+@pytest.mark.parametrize("top_max", [5, 1000])
+def test_top_groups_share_an_sm(orc, per_sm, top_max):
+    """Small-alphabet top streams as warps of one CTA, a share of its shared
+    memory each: more and fewer streams than warps, images from the smallest to
+    the largest of the class, and like-sized streams that give up their groups."""
+    import torch
+
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from fqxv_b200.batch import Codec
+
+    rng = np.random.default_rng(per_sm)
+    sizes = [70_000 - 4_001 * i for i in range(7)]
+    blocks = [_iid(rng, _symbols(rng, nsym), n) for nsym in (2, 5, 6, 13, 15, 31) for n in sizes]
+    blocks += [_cycle(rng, _symbols(rng, 14), 70_000)]
+    streams = [orc.encode(b.tobytes(), 1) for b in blocks]
+    lens = np.array([len(s) for s in streams], np.uint64)
+    spans = np.stack([np.concatenate([[0], np.cumsum(lens)[:-1]]).astype(np.uint64), lens], 1)
+    olens = np.array([len(b) for b in blocks], np.uint64)
+    out_spans = np.stack([np.concatenate([[0], np.cumsum(olens)[:-1]]).astype(np.uint64), olens], 1)
+    d_src = torch.from_numpy(np.frombuffer(b"".join(streams), np.uint8).copy()).to("cuda")
+    codec = Codec(0)
+    try:
+        for name, v in (("o1_top_exclusive", 1), ("o1_top_latency_pct", 0), ("o1_top_max", top_max),
+                        ("o1_top_small_per_sm", per_sm)):
+            codec.set_param(name, v)
+        out, _, status = codec.decode_batch(d_src, spans, out_spans)
+        assert (status == 0).all()
+        assert np.array_equal(out.cpu().numpy(), np.concatenate(blocks))
+    finally:
+        codec.close()
