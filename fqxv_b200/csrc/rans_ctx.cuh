@@ -130,8 +130,9 @@ struct Tuning {
     int64_t cta_cap_o0 = 32, cta_cap_o1_small = 32, cta_cap_o1_wide = 32, cta_cap_o1_four = 8,
             cta_cap_o1_global = 32;
     // the same for the one-warp classes outside the top groups when a batch
-    // has top groups
-    int64_t cta_cap_o1_small_topped = 4, cta_cap_o1_wide_topped = 3;
+    // has top groups (wide at 3, 6: mixed batches of 2048 to 4096 blocks 37.0,
+    // 51.9, 47.5, 40.2 ms and 34.6, 44.8, 46.3, 40.0)
+    int64_t cta_cap_o1_small_topped = 4, cta_cap_o1_wide_topped = 6;
     // table-image sizes cutting the other dense wide-alphabet streams into
     // launch groups (a launch's shared memory is its largest member's)
     int64_t dense_edge_small = 40 << 10, dense_edge_large = 80 << 10;
