@@ -109,6 +109,23 @@ __host__ __device__ inline uint32_t enc_map(uint32_t v, const EncStep &e) {
     return v + (e.pack >> 17) + q * ((e.pack >> 5) & 0xfffu);
 }
 
+// ---- runs of fast decode rounds ---------------------------------------------
+// Groups of G rounds, from round r on, that need no check of the words left:
+// all their symbols are there (below round full), and their words (32 a round
+// at most), with the 64 that a decoder's window may look ahead, end before
+// navail. A run follows its word position in 32 bits, so it takes 2^31 words
+// at most.
+constexpr int64_t kRunRounds = (int64_t)1 << 26;
+template <int G>
+__host__ __device__ __forceinline__ int64_t fast_groups(uint64_t navail, uint64_t wp, uint64_t full, uint64_t r) {
+    const int64_t spare = (int64_t)navail - (int64_t)wp - 64;
+    int64_t groups = spare > 0 ? spare / (32 * G) : 0;
+    const int64_t left = r < full ? (int64_t)(full - r) / G : 0;
+    if (groups > left) groups = left;
+    if (groups > kRunRounds / G) groups = kRunRounds / G;
+    return groups;
+}
+
 // Normalise m (<= 256) counts, held in ascending symbol order, into
 // frequencies summing to 4096 with the reference's rounding and tie rules
 // (crates/fqxv-rans/src/model.rs:213-264):

@@ -29,6 +29,7 @@
 #include <mutex>
 #include <type_traits>
 
+#include "../../include/fqxv_rans_gpu_testing.h"
 #include "rans_common.cuh"
 #include "rans_internal.cuh"
 
@@ -756,10 +757,7 @@ __global__ void __launch_bounds__(32, 1)
         while (status == FQXV_RANS_OK && r < rounds) {
             // A group of G full rounds takes at most 32 G words and its window
             // reads 32 ahead, so `groups` of them cannot run out of words.
-            const int64_t spare = (int64_t)navail - (int64_t)wp - 64;
-            int64_t groups = spare > 0 ? spare / (32 * G) : 0;
-            const int64_t left = r < full ? (int64_t)(full - r) / G : 0;
-            if (groups > left) groups = left;
+            int64_t groups = fast_groups<G>(navail, wp, full, r);
             if (r == 0 || groups <= 0) {
                 if (!o0_general_round(x, P, r, n, R, wp, navail, out, lt)) status = FQXV_RANS_E_TRUNCATED;
                 r++;
@@ -882,10 +880,7 @@ __device__ __forceinline__ int o1_rounds(DecStream &S, WordRing<Col> &R, uint8_t
     uint64_t r = 0;
     int status = FQXV_RANS_OK;
     while (r < rounds && status == FQXV_RANS_OK) {
-        const int64_t spare = (int64_t)navail - (int64_t)wp - 64;
-        int64_t cnt = spare > 0 ? spare / 32 : 0;
-        const int64_t left_full = r < full ? (int64_t)(full - r) : 0;
-        if (cnt > left_full) cnt = left_full;
+        const int64_t cnt = fast_groups<1>(navail, wp, full, r);
         R.advance(wp);
         if (r == 0 || cnt <= 0) {
             // careful round (scalar.rs:202-215 in order)
@@ -1195,10 +1190,7 @@ __device__ __forceinline__ int relay_stream(RelayShared &sh, DecStream &S, const
         if (w == 0) {
             int64_t cnt = 0;
             while (r < rounds && status == FQXV_RANS_OK) {
-                const int64_t spare = (int64_t)navail - (int64_t)wp - 64;
-                cnt = spare > 0 ? spare / 32 : 0;
-                const int64_t left_full = r < full ? (int64_t)(full - r) : 0;
-                if (cnt > left_full) cnt = left_full;
+                cnt = fast_groups<1>(navail, wp, full, r);
                 if (r != 0 && cnt > 0) break;
                 cnt = 0;
                 R.advance(wp);
@@ -1939,3 +1931,7 @@ void launch_dec_run(int cls, const uint8_t *src, DecStream *streams, const uint3
 }
 
 }  // namespace fqxv
+
+extern "C" int64_t fqxv_rans_test_fast_rounds(uint64_t navail, uint64_t wp, uint64_t full, uint64_t r) {
+    return fqxv::fast_groups<1>(navail, wp, full, r);
+}

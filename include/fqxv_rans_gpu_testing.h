@@ -33,6 +33,11 @@ int fqxv_rans_ctx_test_set_wait_polls(fqxv_rans_ctx *ctx, uint32_t polls);
  * FQXV_RANS_E_INVALID_ARG when the entry does not give back f and f << 20. */
 int fqxv_rans_test_enc_map(uint32_t f, uint32_t cum, const uint32_t *v, size_t n, uint32_t *out);
 
+/* Rounds that a decoder runs in one go, without a check of the words left,
+ * from round r of `full` whole rounds and word wp of navail: the kernels'
+ * function, on the host. */
+int64_t fqxv_rans_test_fast_rounds(uint64_t navail, uint64_t wp, uint64_t full, uint64_t r);
+
 #ifdef __cplusplus
 }
 #endif
