@@ -109,6 +109,36 @@ __host__ __device__ inline uint32_t enc_map(uint32_t v, const EncStep &e) {
     return v + (e.pack >> 17) + q * ((e.pack >> 5) & 0xfffu);
 }
 
+// ---- the encoder's symbol chunks ---------------------------------------------
+// A block of n elements of `size` bytes at address `first` has n / 32 whole
+// rounds. The encoder walks them from the last to the first in chunks of
+// kEncChunk rounds, which it copies in aligned granules of 16 bytes; the rounds
+// below the chunks it reads element by element. No granule reaches outside the
+// block: where the lowest whole chunk has no round below it to hold its first
+// granule's lower part, it is left to the rounds below (tail 16), and of the
+// last granule only the part in the block is copied.
+constexpr int kEncChunk = 16;
+struct SymbolPlan {
+    uint64_t top;     // address of the first granule of chunk 0, the highest
+    uint32_t mis;     // bytes of it that lie below the chunk, the same for every chunk
+    uint32_t behind;  // bytes to copy of the granule that holds chunk 0's last `mis` bytes
+    int64_t chunks;   // chunks, each kEncChunk * 32 * size bytes below the one before
+    int64_t tail;     // rounds below them, 0 to kEncChunk
+};
+__host__ __device__ inline SymbolPlan symbol_plan(uint64_t first, uint64_t n, uint32_t size) {
+    const int64_t full = (int64_t)(n / 32);
+    SymbolPlan p;
+    p.top = first + (uint64_t)((full - kEncChunk) * 32) * size;
+    p.mis = (uint32_t)(p.top & 15u);
+    p.top -= p.mis;
+    const uint32_t in_block = p.mis + (uint32_t)(n % 32) * size;
+    p.behind = in_block < 16u ? in_block : 16u;
+    p.chunks = full / kEncChunk;
+    if (p.mis && full && p.chunks * kEncChunk == full) p.chunks--;
+    p.tail = full - p.chunks * kEncChunk;
+    return p;
+}
+
 // ---- runs of fast decode rounds ---------------------------------------------
 // Groups of G rounds, from round r on, that need no check of the words left:
 // all their symbols are there (below round full), and their words (32 a round

@@ -345,8 +345,6 @@ __device__ __forceinline__ bool enc_step(uint32_t &x, const EncStep &e) {
 // 57. Bulk (2048 x 128 KiB), GB/s of input: binned order-0 497 -> 708,
 // full-range order-1 476 -> 535, the latter at 88% of the shared-memory
 // wavefronts (12 a round, most of them 16-byte table entries).
-constexpr int kEncChunk = 16;
-
 struct EncMsg {
     uint16_t word[kEncChunk][32];  // pre-step states' low halves, by round
     uint32_t bits[32];             // lane's emit flags, bit k = round k of the chunk
@@ -484,22 +482,16 @@ constexpr int kStages = 4;
 template <class E>
 struct SymbolRing {
     static constexpr uint32_t kBytes = kEncChunk * 32 * sizeof(E), kStage = kBytes + 16;
-    const uint8_t *top;  // address of the first element of chunk 0
+    const uint8_t *top;  // the plan's
     uint32_t ring;       // shared address
-    uint32_t mis;        // its misalignment, the same for every chunk
+    uint32_t mis, behind;
     int64_t chunks;
 
-    // `first`: element 0 of the block; chunk c holds the rounds
-    // [full - 16 (c + 1), full - 16 c).
-    __device__ SymbolRing(const E *first, int64_t full, uint32_t smem) {
-        chunks = full / kEncChunk;
-        top = reinterpret_cast<const uint8_t *>(first + (full - kEncChunk) * 32);
-        mis = (uint32_t)(uintptr_t)top & 15u;
-        top -= mis;
-        ring = smem;
-    }
+    // Chunk c holds the rounds [full - 16 (c + 1), full - 16 c) of a block of
+    // `full` whole rounds.
+    __device__ SymbolRing(const SymbolPlan &p, uint32_t smem)
+        : top(reinterpret_cast<const uint8_t *>(p.top)), ring(smem), mis(p.mis), behind(p.behind), chunks(p.chunks) {}
     __device__ __forceinline__ uint32_t stage(int64_t c) const { return ring + (uint32_t)(c & (kStages - 1)) * kStage; }
-    // Every copied granule of 16 bytes holds a byte of the chunk.
     __device__ __forceinline__ void fetch(int64_t c) const {
         const uint32_t lane = threadIdx.x & 31;
         if (c < chunks) {
@@ -509,7 +501,8 @@ struct SymbolRing {
             for (uint32_t o = 0; o < kBytes; o += 512)
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + o + 16 * lane), "l"(g + o + 16 * lane));
             if (lane == 0 && mis)
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + kBytes), "l"(g + kBytes));
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d + kBytes), "l"(g + kBytes),
+                             "r"(c == 0 ? behind : 16u));
         }
         asm volatile("cp.async.commit_group;");
     }
@@ -546,7 +539,8 @@ __device__ __forceinline__ uint32_t encode_chain(uint64_t n, const E *__restrict
     const int64_t full = (int64_t)(n / 32);
     const uint32_t rem = (uint32_t)(n % 32);
     auto sym = [&](uint64_t i) -> uint32_t { return (uint32_t)first[i]; };
-    const SymbolRing<E> R(first, full, ring);
+    const SymbolPlan plan = symbol_plan((uint64_t)(uintptr_t)first, n, sizeof(E));
+    const SymbolRing<E> R(plan, ring);
     __syncwarp();  // the last job's reads of the ring are done
 #pragma unroll
     for (int c = 0; c < kStages - 1; c++) R.fetch(c);
@@ -563,7 +557,7 @@ __device__ __forceinline__ uint32_t encode_chain(uint64_t n, const E *__restrict
         pipe.close(m, bits, job, full ? 1 : 3);
         flags = 0;
     }
-    const int64_t tail = full % kEncChunk;  // rounds below the whole chunks
+    const int64_t tail = plan.tail;  // rounds below the whole chunks
     // Symbols of chunk c, whose next chunk is on its way; past the whole
     // chunks, of the rounds below them. `low`: the round below the lowest.
     struct Symbols {
@@ -967,4 +961,15 @@ extern "C" int fqxv_rans_test_enc_map(uint32_t f, uint32_t cum, const uint32_t *
     if (fqxv::enc_freq(e.y) != f || s.keep != (f << 20) - 1u) return FQXV_RANS_E_INVALID_ARG;
     for (size_t i = 0; i < n; i++) out[i] = fqxv::enc_map(v[i], s);
     return FQXV_RANS_OK;
+}
+
+extern "C" void fqxv_rans_test_enc_reads(uint64_t first, uint64_t n, uint32_t size, uint64_t *lo, uint64_t *hi) {
+    // what SymbolRing::fetch copies: the lowest chunk's first granule up, and
+    // chunk 0's last granule with the one behind it
+    const fqxv::SymbolPlan p = fqxv::symbol_plan(first, n, size);
+    *lo = *hi = first;
+    if (p.chunks <= 0) return;
+    const uint64_t bytes = (uint64_t)fqxv::kEncChunk * 32 * size;
+    *lo = p.top - (uint64_t)(p.chunks - 1) * bytes;
+    *hi = p.top + bytes + (p.mis ? p.behind : 0u);
 }

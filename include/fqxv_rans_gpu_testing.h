@@ -33,6 +33,11 @@ int fqxv_rans_ctx_test_set_wait_polls(fqxv_rans_ctx *ctx, uint32_t polls);
  * FQXV_RANS_E_INVALID_ARG when the entry does not give back f and f << 20. */
 int fqxv_rans_test_enc_map(uint32_t f, uint32_t cum, const uint32_t *v, size_t n, uint32_t *out);
 
+/* The addresses [*lo, *hi) that the encoder's chunk copies read of a block of n
+ * elements of `size` bytes at address `first`: the kernel's plan, on the host
+ * (nothing is dereferenced; *lo = *hi = first when it makes no such copy). */
+void fqxv_rans_test_enc_reads(uint64_t first, uint64_t n, uint32_t size, uint64_t *lo, uint64_t *hi);
+
 /* Rounds that a decoder runs in one go, without a check of the words left,
  * from round r of `full` whole rounds and word wp of navail: the kernels'
  * function, on the host. */
