@@ -65,6 +65,30 @@ struct NvtxRange {
     ~NvtxRange() { nvtxRangePop(); }
 };
 
+// At least k streams for the decode launch groups of one kind. The groups of
+// largest streams go on the highest-priority streams, so their CTAs are placed
+// before the rest of the batch fills the SMs.
+cudaError_t ensure_group_streams(fqxv_rans_ctx *ctx, bool top, size_t k) {
+    auto &pool = top ? ctx->aux_top : ctx->aux;
+    if (pool.size() >= k) return cudaSuccess;
+    int lo = 0, hi = 0;
+    if (cudaDeviceGetStreamPriorityRange(&lo, &hi) != cudaSuccess) {
+        cudaGetLastError();
+        lo = hi = 0;
+    }
+    while (pool.size() < k) {
+        fqxv_rans_ctx::GroupStream g;
+        cudaError_t e = cudaStreamCreateWithPriority(&g.s, cudaStreamNonBlocking, top ? hi : lo);
+        if (e == cudaSuccess) {
+            e = cudaEventCreateWithFlags(&g.join, cudaEventDisableTiming);
+            if (e != cudaSuccess) cudaStreamDestroy(g.s);
+        }
+        if (e != cudaSuccess) return e;
+        pool.push_back(g);
+    }
+    return cudaSuccess;
+}
+
 int encode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_span *blocks,
                       size_t nb, int mode, uint8_t *d_dst, uint64_t dst_cap, fqxv_rans_span *out_spans,
                       int32_t *out_orders, int persistent) {
@@ -382,10 +406,11 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
             maxlat[g] = std::max(maxlat[g], (double)ps[i].n * lat_cpb(ps[i]));
             ndmax[g] = std::max(ndmax[g], ps[i].nd);
         }
-        int gcls[kGroups], top_warps[kGroups] = {};
-        uint32_t smem[kGroups];
+        int gcls[kGroups] = {}, top_warps[kGroups] = {};
+        uint32_t smem[kGroups] = {};
         const int64_t four_max = ctx->tune.o1_four_max_streams < 0 ? 3 * ctx->sms : ctx->tune.o1_four_max_streams;
         for (int g = 0; g < kGroups; g++) {
+            if (lists[g].empty()) continue;
             if (g == 0) gcls[g] = kClsO0;
             else if (g == kGroups - 1) gcls[g] = kClsO1Global;
             else if (g == kGroupTiny || g == kGroupTinyTop || g == kGroupTinyAlone) gcls[g] = kClsO1Small;
@@ -411,8 +436,14 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
         int glaunch[kGroups];
         for (int g = 0; g < kGroups; g++) glaunch[g] = g;
         std::stable_sort(glaunch, glaunch + kGroups, [&](int a, int b) { return maxlat[a] > maxlat[b]; });
-        size_t tot = 0;
-        for (int g = 0; g < kGroups; g++) tot += lists[g].size();
+        size_t tot = 0, used = 0, used_top = 0;
+        for (int g = 0; g < kGroups; g++) {
+            tot += lists[g].size();
+            if (!lists[g].empty()) (is_top_group(g) ? used_top : used)++;
+        }
+        CK(ensure_group_streams(ctx, true, used_top));
+        CK(ensure_group_streams(ctx, false, used));
+        used = used_top = 0;
         CK(ctx->d_order.ensure(std::max<size_t>(tot, 1) * 4, s));
         uint32_t *hl = reinterpret_cast<uint32_t *>(hst + szs);
         size_t at = 0, base[kGroups];
@@ -434,7 +465,8 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
             const int stage = cls == kClsO0 ? kStDecO0 : cls == kClsO1Global ? kStDecO1Global
                               : cls == kClsO1Small || cls == kClsO1Mid ? kStDecO1Small : cls == kClsO1Wide ? kStDecO1Wide
                                                                                          : kStDecO1Dense;
-            cudaStream_t as = ctx->aux[g];
+            fqxv_rans_ctx::GroupStream &gs = is_top_group(g) ? ctx->aux_top[used_top++] : ctx->aux[used++];
+            cudaStream_t as = gs.s;
             CK(cudaStreamWaitEvent(as, ctx->ev_fork, 0));
             int per_sm = top_warps[g] ? 1 : dec_blocks_per_sm(cls, smem[g]);
             const Tuning &T = ctx->tune;
@@ -468,8 +500,8 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
                 }
             }
             ctx->timer.bytes[stage] += cbytes[g];
-            CK(cudaEventRecord(ctx->ev_join[g], as));
-            CK(cudaStreamWaitEvent(s, ctx->ev_join[g], 0));
+            CK(cudaEventRecord(gs.join, as));
+            CK(cudaStreamWaitEvent(s, gs.join, 0));
         }
     }
     CK(cudaGetLastError());
@@ -600,18 +632,6 @@ int fqxv_rans_ctx_create(int device, fqxv_rans_ctx **out) {
     if (const char *e = std::getenv("FQXV_RANS_ENC_KEYS")) c->tune.enc_o1_keys = std::strcmp(e, "0") != 0;
     bool ok = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) == cudaSuccess &&
               cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) == cudaSuccess;
-    // The groups of largest streams go on the highest-priority streams, so
-    // their CTAs are placed before the rest of the batch fills the SMs.
-    int prio_lo = 0, prio_hi = 0;
-    if (cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi) != cudaSuccess) {
-        cudaGetLastError();
-        prio_lo = prio_hi = 0;
-    }
-    for (int i = 0; i < kGroups && ok; i++)
-        ok = cudaStreamCreateWithPriority(&c->aux[i], cudaStreamNonBlocking,
-                                          is_top_group(i) ? prio_hi : prio_lo) ==
-                 cudaSuccess &&
-             cudaEventCreateWithFlags(&c->ev_join[i], cudaEventDisableTiming) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         delete c;
@@ -632,10 +652,11 @@ void fqxv_rans_ctx_destroy(fqxv_rans_ctx *ctx) {
     ctx->h_stage.release();
     ctx->h_io.release();
     ctx->timer.release();
-    for (int i = 0; i < kGroups; i++) {
-        if (ctx->aux[i]) cudaStreamDestroy(ctx->aux[i]);
-        if (ctx->ev_join[i]) cudaEventDestroy(ctx->ev_join[i]);
-    }
+    for (auto *pool : {&ctx->aux, &ctx->aux_top})
+        for (auto &g : *pool) {
+            if (g.s) cudaStreamDestroy(g.s);
+            if (g.join) cudaEventDestroy(g.join);
+        }
     if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
     cudaStreamDestroy(ctx->stream);
     delete ctx;

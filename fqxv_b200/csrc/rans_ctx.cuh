@@ -304,8 +304,16 @@ struct fqxv_rans_ctx {
     int device = 0;
     int sms = 148;
     cudaStream_t stream = nullptr;
-    cudaStream_t aux[fqxv::kGroups] = {};   // decode launch groups run side by side
-    cudaEvent_t ev_fork = nullptr, ev_join[fqxv::kGroups] = {};
+    // Decode launch groups run side by side: the k-th top group of a call on
+    // aux_top[k], the k-th other one on aux[k]. A stream and its event are made
+    // when a call first needs them (twelve of them made with every context took
+    // 5.8 ms, most batches have one to four groups).
+    struct GroupStream {
+        cudaStream_t s = nullptr;
+        cudaEvent_t join = nullptr;
+    };
+    std::vector<GroupStream> aux, aux_top;
+    cudaEvent_t ev_fork = nullptr;
     std::mutex mu;
     // encode
     fqxv::DevBuf e_blocks, e_order, e_jobs, e_tbl, e_words, e_hist, e_misc, e_keys;
