@@ -358,9 +358,39 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
         // 256 KiB: 7.7 ms with top groups, 4.3 without; mixed batches of 2048
         // and 4096 blocks, whose first left out take 0.5 to 0.7 of the longest:
         // 35 and 47 ms, 62 and 65 without).
-        if (ntop && ntop < cand.size() && cand[ntop].first > 0.8 * cand[0].first) ntop = 0;
+        const bool alike = ntop && ntop < cand.size() && cand[ntop].first > 0.8 * cand[0].first;
+        if (alike) ntop = 0;
         std::vector<uint8_t> is_top(nb, 0);
         for (size_t k = 0; k < ntop; k++) is_top[cand[k].second] = 1;
+        // The four-warp decoder steps a wide stream's rounds in 529 cycles (the
+        // one-warp decoder in 850) and takes up to three of them to an SM, less
+        // what the SM's other streams leave: full-range blocks of 256 KiB,
+        // four-warp and one-warp: 200 of them 2.65 and 3.88 ms, 444 3.48 and
+        // 3.95, 450 4.48 and 3.95; mixed ones, a quarter wide: 600 2.85 and
+        // 4.0, 1200 4.5 and 5.1, 1500 6.1 and 5.6; an eighth wide: 2000 6.9
+        // and 6.5.
+        auto four_fits = [&](size_t wide, size_t others) {
+            return (double)wide + 0.125 * (double)others <= 3.0 * ctx->sms;
+        };
+        auto is_wide = [&](uint32_t i) { return ps[i].cls == kClsO1Dense && ps[i].nd > kMidMaxNd; };
+        size_t coded = 0, wide = 0;
+        for (size_t i = 0; i < nb; i++)
+            if (ps[i].cls != kClsNone && !is_top[i]) {
+                coded++;
+                wide += is_wide((uint32_t)i);
+            }
+        const bool four = four_fits(wide, coded - wide);
+        // Where all of them are too many but the serial-bound ones alone are
+        // not, these go there, beside the others (128 KiB full-range blocks
+        // with like-sized ones of 1 MiB: 1000 and 150 17.4 -> 10.8 ms, 500 and
+        // 250 17.1 -> 10.7).
+        if (alike && !four && ctx->tune.o1_four_max_streams < 0) {
+            std::vector<uint32_t> longest;
+            for (const auto &c : cand)
+                if (is_wide(c.second) && c.first > 0.5 * cand[0].first) longest.push_back(c.second);
+            if (four_fits(longest.size(), coded - longest.size()))
+                for (uint32_t i : longest) is_top[i] = 1;
+        }
         // Small-alphabet top streams share an SM, top_pack to one, where each
         // takes a tenth longer than alone (names of 1 MiB: 9.4 ms or 8.5).
         // Those that would outlast every other stream by that get an SM each,
@@ -408,7 +438,7 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
         }
         int gcls[kGroups] = {}, top_warps[kGroups] = {};
         uint32_t smem[kGroups] = {};
-        const int64_t four_max = ctx->tune.o1_four_max_streams < 0 ? 3 * ctx->sms : ctx->tune.o1_four_max_streams;
+        const int64_t four_max = ctx->tune.o1_four_max_streams;
         for (int g = 0; g < kGroups; g++) {
             if (lists[g].empty()) continue;
             if (g == 0) gcls[g] = kClsO0;
@@ -416,12 +446,12 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
             else if (g == kGroupTiny || g == kGroupTinyTop || g == kGroupTinyAlone) gcls[g] = kClsO1Small;
             else if (g == kGroupMid || g == kGroupMidTop || g == kGroupMidAlone) gcls[g] = kClsO1Mid;
             else if (g == kGroupFourTop) gcls[g] = kClsO1Dense;
-            else gcls[g] = (int64_t)nb <= four_max ? kClsO1Dense : kClsO1Wide;
+            else gcls[g] = (four_max < 0 ? four : (int64_t)lists[g].size() < four_max) ? kClsO1Dense : kClsO1Wide;
             smem[g] = dec_smem_bytes(gcls[g], tmax[g], ndmax[g]);
             // The groups of largest streams: one CTA per SM, alone on it. One
             // of small alphabets takes up to top_pack streams, as far as
             // their tables fit.
-            if (is_top_group(g) && ctx->tune.o1_top_exclusive) {
+            if (ntop && is_top_group(g) && ctx->tune.o1_top_exclusive) {
                 if (g == kGroupTinyTop || g == kGroupMidTop) {
                     const uint32_t all = dec_exclusive_smem(gcls[g], true);
                     top_warps[g] = (int)std::min<int64_t>(top_pack, all / smem[g]);

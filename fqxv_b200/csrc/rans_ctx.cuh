@@ -105,10 +105,10 @@ const char *const kStageNames[kStages] = {"enc_model", "enc_run", "enc_select_sc
 // them.
 struct Tuning {
     // Order-1 streams of more than kMidMaxNd symbols with shared-memory
-    // tables: batches of at most this many streams send them to the four-warp
-    // decoder, larger ones (the top group aside) to the one-warp decoder. -1:
-    // three to an SM (full-range blocks of 256 KiB, four-warp and one-warp:
-    // 200 of them 2.65 and 3.88 ms, 444 of them 3.48 and 3.95, 592 4.4 and 4.3).
+    // tables: a launch group of fewer than this many goes to the four-warp
+    // decoder, larger groups (the top group aside) to the one-warp decoder.
+    // -1: by how many such streams the batch has to an SM, less for its other
+    // streams (decode_batch_impl).
     int64_t o1_four_max_streams = -1;
     // Order-1 streams whose serial decode alone outlasts o1_top_latency_pct %
     // of the batch's throughput-bound time -- the o1_top_max longest of them

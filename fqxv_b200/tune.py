@@ -21,10 +21,11 @@ reference's only run-time choice is its SIMD backend
                         small group; its longest take an SM each
   enc_o1_keys           order-1 encode reads per-position table indices stored
                         by the model kernel (1) or derives them (0)
-  o1_four_max_streams   batches of at most this many streams send wide-
-                        alphabet order-1 streams to the four-warp decoder
-                        (lower latency per stream), larger ones to the
-                        one-warp decoder (more streams per SM)
+  o1_four_max_streams   below this many wide-alphabet order-1 streams in a
+                        launch group the four-warp decoder (lower latency per
+                        stream) runs them, else the one-warp decoder (more
+                        streams per SM); -1: by how many there are to an SM
+                        beside the batch's other streams
   cta_cap_o1_small_topped / cta_cap_o1_wide_topped
                         the same outside the top groups of a batch that has
                         them (its largest bulk streams run less contended)
@@ -166,7 +167,7 @@ def sweep(reps: int = 3) -> dict:
     pick("o1_top_latency_pct", (25, 50, 75, 100, 150, 100000), score)
     pick("o1_top_max", (sms // 4, sms // 2, 3 * sms // 4, sms), score)
     pick("o1_top_small_per_sm", (1, 2, 4), score)
-    pick("o1_four_max_streams", (0, sms // 2, sms, 2 * sms, 3 * sms, 4 * sms, 1 << 30), score)
+    pick("o1_four_max_streams", (-1, 0, sms // 2, sms, 2 * sms, 3 * sms, 4 * sms, 1 << 30), score)
     # one-warp CTAs per SM outside the top groups, when a batch has them
     pick("cta_cap_o1_small_topped", (2, 4, 8, 16), lambda: bm.decode_gbs(reps))
     pick("cta_cap_o1_wide_topped", (2, 3, 4, 6), lambda: bm.decode_gbs(reps))

@@ -251,6 +251,10 @@ int fqxv_rans_encode_noalloc(const uint8_t *d_src, size_t n, int order, uint8_t 
  *   dense_edge_small, dense_edge_large,
  *   enc_run_ctas_per_sm, enc_run_ctas_per_sm_uniform, enc_o1_keys,
  *   host_enc_chunks, host_dec_chunks, host_in_place, host_out_mirror.
+ * o1_four_max_streams is the size below which a launch group of wide-alphabet
+ * order-1 streams goes to the four-warp decoder (-1: the library's rule, from
+ * the batch's streams per SM). enc_run_ctas_per_sm counts an SM's encode jobs
+ * by fours, as they once shared a CTA.
  * Unknown names and out-of-range values: FQXV_RANS_E_INVALID_ARG. Output
  * bytes never depend on them. */
 int fqxv_rans_ctx_set_param(fqxv_rans_ctx *ctx, const char *name, int64_t value);
