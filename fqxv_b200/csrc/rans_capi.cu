@@ -366,7 +366,7 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
         // one-warp decoder in 850) and takes up to three of them to an SM, less
         // what the SM's other streams leave: full-range blocks of 256 KiB,
         // four-warp and one-warp: 200 of them 2.65 and 3.88 ms, 444 3.48 and
-        // 3.95, 450 4.48 and 3.95; mixed ones, a quarter wide: 600 2.85 and
+        // 3.78, 450 4.48 and 3.78; mixed ones, a quarter wide: 600 2.85 and
         // 4.0, 1200 4.5 and 5.1, 1500 6.1 and 5.6; an eighth wide: 2000 6.9
         // and 6.5.
         auto four_fits = [&](size_t wide, size_t others) {
