@@ -435,99 +435,12 @@ int rebuild_names(uint64_t n_records, const uint8_t *counts, uint64_t ncounts, c
     return FQXV_RANS_OK;
 }
 
-}  // namespace
-
-extern "C" {
-
-int fqxv_tok_encode_host(fqxv_rans_ctx *ctx, const uint8_t *h_names, const fqxv_rans_span *name_spans,
-                         size_t nnames, const fqxv_rans_span *blocks, size_t nblocks, uint8_t *h_dst,
-                         uint64_t cap, fqxv_rans_span *out, uint64_t *needed) {
-    if (!ctx || (nblocks && (!blocks || !out)) || (nnames && (!name_spans || !h_names))) return FQXV_RANS_E_INVALID_ARG;
-    for (size_t b = 0; b < nblocks; b++)
-        if (blocks[b].offset > nnames || blocks[b].length > nnames - blocks[b].offset) return FQXV_RANS_E_INVALID_ARG;
-    std::vector<BlockRoles> roles(nblocks);
-    parallel_for(nblocks, [&](size_t b) {
-        build_roles(h_names, name_spans, blocks[b].offset, blocks[b].length, roles[b]);
-    });
-    // every role stream of every block in one arena, coded in one pass
-    size_t ns = 0;
-    uint64_t raw_total = 0;
-    for (auto &B : roles) {
-        ns += B.len.size();
-        raw_total += B.raw.size();
-    }
-    std::vector<uint8_t> arena(std::max<uint64_t>(raw_total, 1));
-    std::vector<fqxv_rans_span> sp(ns), coded(ns);
-    uint64_t pos = 0, code_cap = 0;
-    size_t k = 0;
-    for (auto &B : roles) {
-        if (!B.raw.empty()) std::memcpy(arena.data() + pos, B.raw.data(), B.raw.size());
-        uint64_t o = pos;
-        for (uint64_t l : B.len) {
-            sp[k++] = fqxv_rans_span{o, l};
-            o += l;
-            code_cap += 9 + 512 + 128 + 2 * l;  // the order-0 bound covers the smaller of the two
-        }
-        pos += B.raw.size();
-    }
-    std::vector<uint8_t> cbuf(std::max<uint64_t>(code_cap, 1));
-    if (ns) {
-        const int st = fqxv_rans_encode_batch_host(ctx, arena.data(), sp.data(), ns, FQXV_RANS_BEST_TIE0,
-                                                   cbuf.data(), code_cap, coded.data(), nullptr);
-        if (st) return st;
-    }
-    // payloads: [1][varint n][8 x (varint len, stream)][64 x (varint width, planes)]
-    std::vector<uint64_t> psize(nblocks);
-    std::vector<size_t> first(nblocks + 1, 0);
-    for (size_t b = 0; b < nblocks; b++) first[b + 1] = first[b] + roles[b].len.size();
-    auto vlen = [](uint64_t v) {
-        uint64_t n = 1;
-        while (v >>= 7) n++;
-        return n;
-    };
-    uint64_t total = 0;
-    for (size_t b = 0; b < nblocks; b++) {
-        uint64_t t = 1 + vlen(roles[b].n_records);
-        for (size_t s = first[b]; s < first[b + 1]; s++) t += vlen(coded[s].length) + coded[s].length;
-        for (int c = 0; c < kCols; c++) t += vlen(roles[b].width[c]);
-        psize[b] = t;
-        total += t;
-    }
-    if (needed) *needed = total;
-    if (total > cap || (total && !h_dst)) return FQXV_RANS_E_DST_TOO_SMALL;
-    std::vector<uint64_t> start(nblocks);
-    for (size_t b = 0, o = 0; b < nblocks; b++) {
-        start[b] = o;
-        o += psize[b];
-    }
-    parallel_for(nblocks, [&](size_t b) {
-        std::vector<uint8_t> p;
-        p.reserve(psize[b]);
-        p.push_back(kVersion);
-        put_varint(p, roles[b].n_records);
-        auto stream = [&](size_t s) {
-            put_varint(p, coded[s].length);
-            p.insert(p.end(), cbuf.data() + coded[s].offset, cbuf.data() + coded[s].offset + coded[s].length);
-        };
-        size_t s = first[b];
-        for (int f = 0; f < kFlat; f++) stream(s++);
-        for (int c = 0; c < kCols; c++) {
-            put_varint(p, roles[b].width[c]);
-            for (int q = 0; q < roles[b].width[c]; q++) stream(s++);
-        }
-        std::memcpy(h_dst + start[b], p.data(), p.size());
-        out[b] = fqxv_rans_span{start[b], p.size()};
-    });
-    return FQXV_RANS_OK;
-}
-
-int fqxv_tok_decode_host(fqxv_rans_ctx *ctx, const uint8_t *h_src, const fqxv_rans_span *payloads, size_t nblocks,
-                         uint8_t *h_names, uint64_t names_cap, fqxv_rans_span *name_spans, uint64_t spans_cap,
-                         fqxv_rans_span *blocks, int32_t *status, uint64_t *names_needed, uint64_t *spans_needed) {
-    if (!ctx || (nblocks && (!payloads || !h_src || !blocks || !status))) return FQXV_RANS_E_INVALID_ARG;
+// The names and status of every payload in `out`; the return value is not a
+// block's status but the coder's own failure.
+int decode_payloads(fqxv_rans_ctx *ctx, const uint8_t *h_src, const fqxv_rans_span *payloads, size_t nblocks,
+                    std::vector<BlockOut> &out) {
     std::vector<Frame> F(nblocks);
     parallel_for(nblocks, [&](size_t b) { frame_payload(h_src + payloads[b].offset, payloads[b].length, F[b]); });
-    std::vector<BlockOut> out(nblocks);
     // pass 1: the flat and op-run streams (decode_bounded by max_out, lib.rs:107-110)
     DecodeList d1;
     std::vector<size_t> flat_first(nblocks);
@@ -669,18 +582,23 @@ int fqxv_tok_decode_host(fqxv_rans_ctx *ctx, const uint8_t *h_src, const fqxv_ra
             o.name_len.clear();
         }
     });
-    uint64_t nb_bytes = 0, nb_names = 0;
+    return FQXV_RANS_OK;
+}
+
+void output_size(const std::vector<BlockOut> &out, uint64_t &bytes, uint64_t &names) {
+    bytes = names = 0;
     for (auto &o : out) {
-        nb_bytes += o.bytes.size();
-        nb_names += o.name_len.size();
+        bytes += o.bytes.size();
+        names += o.name_len.size();
     }
-    if (names_needed) *names_needed = nb_bytes;
-    if (spans_needed) *spans_needed = nb_names;
-    if (nb_bytes > names_cap || nb_names > spans_cap || (nb_bytes && !h_names) || (nb_names && !name_spans))
-        return FQXV_RANS_E_DST_TOO_SMALL;
+}
+
+// Everything into the caller's buffers; returns the first failed block's status.
+int write_names(const std::vector<BlockOut> &out, uint8_t *h_names, fqxv_rans_span *name_spans,
+                fqxv_rans_span *blocks, int32_t *status) {
     int first = FQXV_RANS_OK;
     uint64_t bo = 0, no = 0;
-    for (size_t b = 0; b < nblocks; b++) {
+    for (size_t b = 0; b < out.size(); b++) {
         const BlockOut &o = out[b];
         status[b] = o.status;
         if (o.status && first == FQXV_RANS_OK) first = o.status;
@@ -692,6 +610,124 @@ int fqxv_tok_decode_host(fqxv_rans_ctx *ctx, const uint8_t *h_src, const fqxv_ra
         }
     }
     return first;
+}
+
+}  // namespace
+
+extern "C" {
+
+int fqxv_tok_encode_host(fqxv_rans_ctx *ctx, const uint8_t *h_names, const fqxv_rans_span *name_spans,
+                         size_t nnames, const fqxv_rans_span *blocks, size_t nblocks, uint8_t *h_dst,
+                         uint64_t cap, fqxv_rans_span *out, uint64_t *needed) {
+    if (!ctx || (nblocks && (!blocks || !out)) || (nnames && (!name_spans || !h_names))) return FQXV_RANS_E_INVALID_ARG;
+    for (size_t b = 0; b < nblocks; b++)
+        if (blocks[b].offset > nnames || blocks[b].length > nnames - blocks[b].offset) return FQXV_RANS_E_INVALID_ARG;
+    std::vector<BlockRoles> roles(nblocks);
+    parallel_for(nblocks, [&](size_t b) {
+        build_roles(h_names, name_spans, blocks[b].offset, blocks[b].length, roles[b]);
+    });
+    // every role stream of every block in one arena, coded in one pass
+    size_t ns = 0;
+    uint64_t raw_total = 0;
+    for (auto &B : roles) {
+        ns += B.len.size();
+        raw_total += B.raw.size();
+    }
+    std::vector<uint8_t> arena(std::max<uint64_t>(raw_total, 1));
+    std::vector<fqxv_rans_span> sp(ns), coded(ns);
+    uint64_t pos = 0, code_cap = 0;
+    size_t k = 0;
+    for (auto &B : roles) {
+        if (!B.raw.empty()) std::memcpy(arena.data() + pos, B.raw.data(), B.raw.size());
+        uint64_t o = pos;
+        for (uint64_t l : B.len) {
+            sp[k++] = fqxv_rans_span{o, l};
+            o += l;
+            code_cap += 9 + 512 + 128 + 2 * l;  // the order-0 bound covers the smaller of the two
+        }
+        pos += B.raw.size();
+    }
+    std::vector<uint8_t> cbuf(std::max<uint64_t>(code_cap, 1));
+    if (ns) {
+        const int st = fqxv_rans_encode_batch_host(ctx, arena.data(), sp.data(), ns, FQXV_RANS_BEST_TIE0,
+                                                   cbuf.data(), code_cap, coded.data(), nullptr);
+        if (st) return st;
+    }
+    // payloads: [1][varint n][8 x (varint len, stream)][64 x (varint width, planes)]
+    std::vector<uint64_t> psize(nblocks);
+    std::vector<size_t> first(nblocks + 1, 0);
+    for (size_t b = 0; b < nblocks; b++) first[b + 1] = first[b] + roles[b].len.size();
+    auto vlen = [](uint64_t v) {
+        uint64_t n = 1;
+        while (v >>= 7) n++;
+        return n;
+    };
+    uint64_t total = 0;
+    for (size_t b = 0; b < nblocks; b++) {
+        uint64_t t = 1 + vlen(roles[b].n_records);
+        for (size_t s = first[b]; s < first[b + 1]; s++) t += vlen(coded[s].length) + coded[s].length;
+        for (int c = 0; c < kCols; c++) t += vlen(roles[b].width[c]);
+        psize[b] = t;
+        total += t;
+    }
+    if (needed) *needed = total;
+    if (total > cap || (total && !h_dst)) return FQXV_RANS_E_DST_TOO_SMALL;
+    std::vector<uint64_t> start(nblocks);
+    for (size_t b = 0, o = 0; b < nblocks; b++) {
+        start[b] = o;
+        o += psize[b];
+    }
+    parallel_for(nblocks, [&](size_t b) {
+        std::vector<uint8_t> p;
+        p.reserve(psize[b]);
+        p.push_back(kVersion);
+        put_varint(p, roles[b].n_records);
+        auto stream = [&](size_t s) {
+            put_varint(p, coded[s].length);
+            p.insert(p.end(), cbuf.data() + coded[s].offset, cbuf.data() + coded[s].offset + coded[s].length);
+        };
+        size_t s = first[b];
+        for (int f = 0; f < kFlat; f++) stream(s++);
+        for (int c = 0; c < kCols; c++) {
+            put_varint(p, roles[b].width[c]);
+            for (int q = 0; q < roles[b].width[c]; q++) stream(s++);
+        }
+        std::memcpy(h_dst + start[b], p.data(), p.size());
+        out[b] = fqxv_rans_span{start[b], p.size()};
+    });
+    return FQXV_RANS_OK;
+}
+
+int fqxv_tok_decode_host(fqxv_rans_ctx *ctx, const uint8_t *h_src, const fqxv_rans_span *payloads, size_t nblocks,
+                         uint8_t *h_names, uint64_t names_cap, fqxv_rans_span *name_spans, uint64_t spans_cap,
+                         fqxv_rans_span *blocks, int32_t *status, uint64_t *names_needed, uint64_t *spans_needed) {
+    if (!ctx || (nblocks && (!payloads || !h_src || !blocks || !status))) return FQXV_RANS_E_INVALID_ARG;
+    std::vector<BlockOut> out(nblocks);
+    const int r = decode_payloads(ctx, h_src, payloads, nblocks, out);
+    if (r) return r;
+    uint64_t nb_bytes, nb_names;
+    output_size(out, nb_bytes, nb_names);
+    if (names_needed) *names_needed = nb_bytes;
+    if (spans_needed) *spans_needed = nb_names;
+    if (nb_bytes > names_cap || nb_names > spans_cap || (nb_bytes && !h_names) || (nb_names && !name_spans))
+        return FQXV_RANS_E_DST_TOO_SMALL;
+    return write_names(out, h_names, name_spans, blocks, status);
+}
+
+int fqxv_tok_decode_host_alloc(fqxv_rans_ctx *ctx, const uint8_t *h_src, const fqxv_rans_span *payloads,
+                               size_t nblocks, fqxv_tok_alloc_fn alloc, void *user, fqxv_rans_span *blocks,
+                               int32_t *status) {
+    if (!ctx || !alloc || (nblocks && (!payloads || !h_src || !blocks || !status))) return FQXV_RANS_E_INVALID_ARG;
+    std::vector<BlockOut> out(nblocks);
+    const int r = decode_payloads(ctx, h_src, payloads, nblocks, out);
+    if (r) return r;
+    uint64_t nb_bytes, nb_names;
+    output_size(out, nb_bytes, nb_names);
+    uint8_t *h_names = nullptr;
+    fqxv_rans_span *name_spans = nullptr;
+    if (alloc(user, nb_bytes, nb_names, &h_names, &name_spans) || (nb_bytes && !h_names) || (nb_names && !name_spans))
+        return FQXV_RANS_E_OUT_OF_MEMORY;
+    return write_names(out, h_names, name_spans, blocks, status);
 }
 
 }  // extern "C"

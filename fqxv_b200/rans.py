@@ -86,6 +86,11 @@ X_MALFORMED = 9
 STREAM_STATUSES = MALFORMED | {TIMEOUT, X_MALFORMED}
 
 
+# fqxv_tok_alloc_fn (include/fqxv_tok_gpu.h)
+TokAlloc = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.c_uint64, ctypes.c_uint64,
+                            ctypes.POINTER(ctypes.c_void_p), ctypes.POINTER(ctypes.c_void_p))
+
+
 def lib_path() -> str:
     return _build.LIB
 
@@ -151,6 +156,7 @@ def lib() -> ctypes.CDLL:
                                            ctypes.POINTER(ctypes.c_uint64)]
         L.fqxv_tok_decode_host.argtypes = [vp, u8p, u8p, sz, u8p, ctypes.c_uint64, u8p, ctypes.c_uint64, u8p, u8p,
                                            ctypes.POINTER(ctypes.c_uint64), ctypes.POINTER(ctypes.c_uint64)]
+        L.fqxv_tok_decode_host_alloc.argtypes = [vp, u8p, u8p, sz, TokAlloc, vp, u8p, u8p]
         # put_stream framing and the permutation planes (include/fqxv_streams_gpu.h)
         L.fqxv_put_streams_host.argtypes = [vp, u8p, u8p, sz, u8p, ctypes.c_uint64, u8p,
                                             ctypes.POINTER(ctypes.c_uint64)]

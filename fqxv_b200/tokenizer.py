@@ -88,27 +88,27 @@ def decode_blocks(payloads, device: int = 0, raise_on_error: bool = True):
     L = rans.lib()
     blocks = np.zeros((max(n, 1), 2), dtype=np.uint64)
     status = np.zeros(max(n, 1), dtype=np.int32)
-    nb, ns = ctypes.c_uint64(0), ctypes.c_uint64(0)
-    # Untouched memory costs nothing; a buffer that turns out too small costs
-    # a second decode (sequencer names shrink 10 to 20 times). Large calls
-    # start from less.
-    names_cap = min(64 * arena.size, max(8 * arena.size, 1 << 28)) + 4096
-    spans_cap = min(4 * arena.size, max(arena.size, 1 << 24)) + 64
-    for _ in range(2):
-        h_names = np.empty(max(names_cap, 1), dtype=np.uint8)
-        nsp = np.empty((max(spans_cap, 1), 2), dtype=np.uint64)
-        st = L.fqxv_tok_decode_host(c._h, arena.ctypes.data, psp.ctypes.data, n, h_names.ctypes.data, names_cap,
-                                    nsp.ctypes.data, spans_cap, blocks.ctypes.data, status.ctypes.data,
-                                    ctypes.byref(nb), ctypes.byref(ns))
-        if st == 17 and (nb.value > names_cap or ns.value > spans_cap):
-            names_cap, spans_cap = max(nb.value, 1), max(ns.value, 1)
-            continue
-        break
+    bufs, failed = [], []
+
+    def alloc(_, nbytes, nnames, names_p, spans_p):
+        try:
+            bufs[:] = np.empty(nbytes, dtype=np.uint8), np.empty((nnames, 2), dtype=np.uint64)
+        except BaseException as e:
+            failed.append(e)
+            return 1
+        names_p[0], spans_p[0] = (a.ctypes.data for a in bufs)
+        return 0
+
+    st = L.fqxv_tok_decode_host_alloc(c._h, arena.ctypes.data, psp.ctypes.data, n, rans.TokAlloc(alloc), None,
+                                      blocks.ctypes.data, status.ctypes.data)
+    if failed:
+        raise failed[0]
     if st and st not in TOK_STATUSES and st not in rans.MALFORMED:
         _raise(st)
     # One bytes object, sliced by plain ints: a numpy slice and copy per name
     # took most of a call (128,000 names).
-    text = h_names[:nb.value].tobytes()
+    h_names, nsp = bufs
+    text = h_names.tobytes()
     out = []
     for b in range(n):
         f, k = int(blocks[b, 0]), int(blocks[b, 1])

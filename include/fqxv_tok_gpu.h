@@ -66,6 +66,17 @@ int fqxv_tok_decode_host(fqxv_rans_ctx *ctx, const uint8_t *h_src, const fqxv_ra
                          uint8_t *h_names, uint64_t names_cap, fqxv_rans_span *name_spans, uint64_t spans_cap,
                          fqxv_rans_span *blocks, int32_t *status, uint64_t *names_needed, uint64_t *spans_needed);
 
+/* The same with buffers of the names' own size: when the sizes are known, and
+ * once per call that decodes, alloc(user, names_bytes, nnames, &h_names,
+ * &name_spans) is called on this thread and sets both pointers (either may stay
+ * NULL when its size is 0). If it returns non-zero nothing is written and
+ * FQXV_RANS_E_OUT_OF_MEMORY is returned. */
+typedef int (*fqxv_tok_alloc_fn)(void *user, uint64_t names_bytes, uint64_t nnames, uint8_t **h_names,
+                                 fqxv_rans_span **name_spans);
+int fqxv_tok_decode_host_alloc(fqxv_rans_ctx *ctx, const uint8_t *h_src, const fqxv_rans_span *payloads,
+                               size_t nblocks, fqxv_tok_alloc_fn alloc, void *user, fqxv_rans_span *blocks,
+                               int32_t *status);
+
 #ifdef __cplusplus
 }
 #endif
