@@ -538,8 +538,9 @@ struct WordRing {
         ring = reinterpret_cast<Elem *>(r);
         reset(0);
     }
-    // Keep the 3 kSegWords words from word index wp on resident
-    // (warp-uniform).
+    // Brings the ring to word index wp, from anywhere before it (warp-uniform).
+    // After a jump of more than a segment the rest of wp's segment and the two
+    // behind it are resident; follow() adds the next.
     __device__ __forceinline__ void advance(uint64_t wp) {
         const uint32_t seg = (uint32_t)((lead + wp) / kSegWords);
         while (seg >= next_seg - 3) {
@@ -556,6 +557,7 @@ struct WordRing {
     }
     // The same between groups of rounds, where the position has moved by a few
     // segments at most: 32-bit arithmetic, and one test when nothing is due.
+    // 3 kSegWords words from w32 on are resident afterwards.
     __device__ __forceinline__ void follow(uint32_t w32) {
         while ((int32_t)(lead + w32 - kSegWords * (next_seg - 3)) >= 0) {
             __syncwarp();
@@ -753,7 +755,7 @@ __global__ void __launch_bounds__(32, 1)
         // the 64-bit checks between groups (256 KiB of binned quality).
         uint64_t r = 0;
         constexpr int G = 8;  // rounds per branch-free group
-        static_assert(32 * G + 64 <= 3 * kSegWords, "a group's words are resident after one ring advance");
+        static_assert(32 * G + 64 <= 3 * kSegWords, "a group's words are resident once the ring has followed");
         while (status == FQXV_RANS_OK && r < rounds) {
             // A group of G full rounds takes at most 32 G words and its window
             // reads 32 ahead, so `groups` of them cannot run out of words.
@@ -870,7 +872,7 @@ __device__ __forceinline__ void take_word(uint2 q, uint32_t srcl, uint32_t v, ui
 // branched around (1800 full-range blocks of 256 KiB 11.8 -> 11.3 ms, with the
 // shorter trial; 512 binned ones 3.05 -> 2.97, 700 ONT ones 6.79 -> 6.58).
 constexpr int kO1Group = 8;
-static_assert(32 * kO1Group + 64 <= 3 * kSegWords, "a group's words are resident after one ring advance");
+static_assert(32 * kO1Group + 64 <= 3 * kSegWords, "a group's words are resident once the ring has followed");
 
 template <class Col, class D>
 __device__ __forceinline__ int o1_rounds(DecStream &S, WordRing<Col> &R, uint8_t *__restrict__ out, uint32_t lt,
@@ -1072,11 +1074,11 @@ __device__ __forceinline__ void relay_rounds(RelayShared &sh, const DenseImage &
     const uint32_t c0 = min((uint32_t)lane, I.dead), c1 = HI ? min((uint32_t)lane + 32u, I.dead) : 0u;
     uint32_t cb = C.look(x & (kTotFreq - 1));
     uint32_t pos = (uint32_t)wp;
+    R.advance(wp);
     op += 8 * w + k;
-    for (int64_t i = 0; i < cnt; i += 8) {
-        wp += (uint32_t)(pos - (uint32_t)wp);
-        R.advance(wp);
-        const int m = (int)(cnt - i < 8 ? cnt - i : 8);
+    for (int64_t i = 0; i < cnt; i += kO1Group) {
+        R.follow(pos);
+        const int m = (int)(cnt - i < kO1Group ? cnt - i : kO1Group);
         for (int g = 0; g < m; g++) {
             const bool first = w == 0 && i + g == 0;
             uint32_t in = din, last, a, b, o[8];
