@@ -362,7 +362,7 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
         if (alike) ntop = 0;
         std::vector<uint8_t> is_top(nb, 0);
         for (size_t k = 0; k < ntop; k++) is_top[cand[k].second] = 1;
-        // The four-warp decoder steps a wide stream's rounds in 529 cycles (the
+        // The four-warp decoder steps a wide stream's rounds in 524 cycles (the
         // one-warp decoder in 850) and takes up to three of them to an SM, less
         // what the SM's other streams leave: full-range blocks of 256 KiB,
         // four-warp and one-warp: 200 of them 2.65 and 3.88 ms, 444 3.48 and
@@ -1095,16 +1095,18 @@ int decode_host_one(fqxv_rans_ctx *ctx, const uint8_t *h_src, const fqxv_rans_sp
                           ? static_cast<uint8_t *>(mapped_device_ptr(h_dst))
                           : nullptr;
     // A slow batch of hundreds of streams also reads its pinned input in
-    // place: each stream's words are fetched 16 bytes a lane, segments ahead
+    // place: each stream's words are fetched 8 bytes a lane, segments ahead
     // of use, at a small share of the link, and the decode starts without
-    // waiting for a copy. Measured on B200: 4103 mixed streams (4 KiB to
-    // 4 MiB) e2e 17.2 -> 21.2 GB/s, but chunks of 16 x 1 MiB order-1 streams
-    // 4.63 -> 4.36, so smaller batches (and single serving requests) keep
-    // the staged copy, issued before this point. "Slow": the decode time,
-    // estimated from the stream headers (the largest stream's serial rounds,
-    // about 320 ns per 32 bytes for order-1 and 80 ns for order-0 on B200,
-    // or the whole batch at the batched rates, about 15 and 300 GB/s), keeps
-    // the output rate under 40 GB/s.
+    // waiting for a copy (staged and in place: 512 x 512 KiB full-range 14.8
+    // and 12.4 ms, 1000 mixed blocks 37.9 and 35.0, 512 binned order-1 8.3 and
+    // 8.0). Chunks of 16 x 1 MiB order-1 streams lost 6% by it, so smaller
+    // batches (and single serving requests) keep the staged copy, issued
+    // before this point. "Slow": an estimate of the decode time from the
+    // stream headers keeps the output rate under 40 GB/s. It weighs the largest
+    // stream's serial rounds at 320 ns per 32 bytes of order-1 and 80 of
+    // order-0, or the whole batch at 15 and 300 GB/s: weights of this choice,
+    // above what the decoders take now (270 and 65 ns), as reading in place
+    // was the faster one wherever they choose it.
     if (!d_in && in_place > 0) d_in = static_cast<const uint8_t *>(mapped_device_ptr(h_src));
     if (!d_in && mirror) {
         double t_lat = 0.0, b0 = 0.0, b1 = 0.0;

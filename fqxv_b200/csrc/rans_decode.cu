@@ -17,12 +17,12 @@
 //      shared-memory ring that the warp refills with 8-byte loads issued a
 //      segment ahead. The stream's tables are staged into shared memory with
 //      one TMA bulk copy (cp.async.bulk + mbarrier, bounded wait).
-//      Order-1 resolves each round's context chain s_i = column_i[s_{i-1}]
-//      exactly, in four segments of eight lanes: the first from the known
-//      context, the other three for every possible incoming context at once,
-//      then three dependent lookups pick the real paths; or, in the one-warp
-//      decoders, by guessing every lane's context from the columns right
-//      below it and checking the guesses.
+//      Order-1 resolves each round's context chain s_i = column_i[s_{i-1}]:
+//      the one-warp decoders guess every lane's context from the columns right
+//      below it and check the guesses, or run every context of four segments
+//      of eight lanes and follow three rows; the four-warp decoder composes
+//      eight columns at a time as functions of a context that is still on its
+//      way.
 // Malformed input never faults: every read of the stream is bounds checked
 // and errors are reported per stream as the reference's Malformed kinds.
 #include <algorithm>
@@ -1029,11 +1029,11 @@ struct DenseImage {
 // What bounds it is a warp's own loop, about 130 instructions, most of them
 // in one dependent chain (a hop to the next warp is ~85 cycles, four a round
 // ~340). One stream, cycles per round: full-range quality (31 or 32 symbols)
-// 529, ONT quality (39) 601, random walk (41) 598; a context 0 that is no
-// symbol once counted, and took the streams of 32 symbols to the wider form's
-// 601. Before, every warp held all 32
-// states, ran a segment's chains from every context and followed three rows
-// of shared memory behind a barrier: 642, 614 and 615.
+// 524, ONT quality (39) 597, random walk (41) 589; a context 0 that is no
+// symbol once counted, and took the streams of 32 symbols to the wider form.
+// Before, every warp held all 32 states, ran a segment's chains from every
+// context and followed three rows of shared memory behind a barrier: 642, 614
+// and 615.
 constexpr int kO1Warps = 4;
 constexpr int kO1Threads = 32 * kO1Warps;
 
@@ -1433,8 +1433,7 @@ struct TinyDecoder : GuessTrust<64> {
 // share one segment, so a round needs eight column shuffles per lane whatever
 // TPL is. Rows go to a double-buffered shared array (rows 0 .. 3 nd - 1, then
 // the DEAD row and a row for lanes without a task) and are resolved after a
-// __syncwarp with three dependent loads, as in the four-warp decoder, but
-// without its barrier or its replicated states.
+// __syncwarp with three dependent loads.
 constexpr int kWideLanes = 10;  // lanes per speculative segment
 
 template <int TPL>

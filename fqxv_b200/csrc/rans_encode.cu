@@ -11,7 +11,7 @@
 //      the rounds from the last to the first, emitting renorm words with a
 //      ballot/popc compaction written back to front into a word scratch.
 //   3. enc_select_scan    encoded sizes, order selection, exclusive scan.
-//   4. enc_pack_kernel    one CTA per block: header, frequency tables, states
+//   4. enc_pack_kernel    eight CTAs per block: header, frequency tables, states
 //      and words written to their compacted place in the output arena.
 // Byte format and arithmetic follow crates/fqxv-rans/src/scalar.rs:29-140 and
 // model.rs:52-264.
@@ -641,6 +641,14 @@ constexpr uint32_t kEncO1SmemNu = 45;
 constexpr uint32_t kEncO1TabBytes = kEncO1StepNu * kEncO1StepNu * 16;
 static_assert(kEncO1SmemNu * kEncO1SmemNu * 8 <= kEncO1TabBytes, "a packed table fits the slice");
 
+// Four CTAs per SM is the register limit; a fourth of its 228 KB of shared
+// memory holds one, with 1 KB that the hardware reserves per CTA.
+static_assert(kEncJobsPerCta * (256 * (sizeof(EncStep) + 1) + 2 * sizeof(EncMsg) +
+                                kStages * SymbolRing<uint16_t>::kStage + kEncO1TabBytes) +
+                      1024 <=
+                  228 * 1024 / 4,
+              "four encode CTAs per SM");
+
 // Warps 0 .. kEncJobsPerCta - 1 are chain warps, the others emit warps, each
 // of the next pair's number, so a pair's two warps sit on two schedulers.
 __global__ void __launch_bounds__(kEncJobsPerCta * 64, 4)
@@ -931,7 +939,6 @@ void launch_enc_run(const uint8_t *src, EncBlock *blocks, const EncJob *jobs, in
         if (dev >= 0 && dev < 256 && !done[dev]) {
             cudaFuncSetAttribute(enc_run_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(kEncJobsPerCta * kEncO1TabBytes));
-            // four CTAs per SM (the register limit) need ~170 KB of shared memory
             cudaFuncSetAttribute(enc_run_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  cudaSharedmemCarveoutMaxShared);
             cudaGetLastError();
