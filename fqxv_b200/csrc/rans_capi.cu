@@ -362,35 +362,6 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
         if (alike) ntop = 0;
         std::vector<uint8_t> is_top(nb, 0);
         for (size_t k = 0; k < ntop; k++) is_top[cand[k].second] = 1;
-        // The four-warp decoder steps a wide stream's rounds in 524 cycles (the
-        // one-warp decoder in 850) and takes up to three of them to an SM, less
-        // what the SM's other streams leave: full-range blocks of 256 KiB,
-        // four-warp and one-warp: 200 of them 2.65 and 3.88 ms, 444 3.48 and
-        // 3.78, 450 4.48 and 3.78; mixed ones, a quarter wide: 600 2.85 and
-        // 4.0, 1200 4.5 and 5.1, 1500 6.1 and 5.6; an eighth wide: 2000 6.9
-        // and 6.5.
-        auto four_fits = [&](size_t wide, size_t others) {
-            return (double)wide + 0.125 * (double)others <= 3.0 * ctx->sms;
-        };
-        auto is_wide = [&](uint32_t i) { return ps[i].cls == kClsO1Dense && ps[i].nd > kMidMaxNd; };
-        size_t coded = 0, wide = 0;
-        for (size_t i = 0; i < nb; i++)
-            if (ps[i].cls != kClsNone && !is_top[i]) {
-                coded++;
-                wide += is_wide((uint32_t)i);
-            }
-        const bool four = four_fits(wide, coded - wide);
-        // Where all of them are too many but the serial-bound ones alone are
-        // not, these go there, beside the others (128 KiB full-range blocks
-        // with like-sized ones of 1 MiB: 1000 and 150 17.4 -> 10.8 ms, 500 and
-        // 250 17.1 -> 10.7).
-        if (alike && !four && ctx->tune.o1_four_max_streams < 0) {
-            std::vector<uint32_t> longest;
-            for (const auto &c : cand)
-                if (is_wide(c.second) && c.first > 0.5 * cand[0].first) longest.push_back(c.second);
-            if (four_fits(longest.size(), coded - longest.size()))
-                for (uint32_t i : longest) is_top[i] = 1;
-        }
         // Small-alphabet top streams share an SM, top_pack to one, where each
         // takes a tenth longer than alone (names of 1 MiB: 9.4 ms or 8.5).
         // Those that would outlast every other stream by that get an SM each,
@@ -409,6 +380,41 @@ int decode_batch_impl(fqxv_rans_ctx *ctx, const uint8_t *d_src, const fqxv_rans_
                 is_top[cand[k].second] = 2;
                 spare -= 1.0 - 1.0 / (double)top_pack;
             }
+        }
+        // The four-warp decoder steps a wide stream's rounds in 524 cycles (the
+        // one-warp decoder in 850) and takes up to three of them to an SM that
+        // no top stream holds, less what the SM's other streams leave: full-range
+        // blocks of 256 KiB, four-warp and one-warp: 200 of them 2.65 and 3.88
+        // ms, 444 3.48 and 3.78, 450 4.48 and 3.78; mixed ones, a quarter wide:
+        // 600 2.85 and 4.0, 1200 4.5 and 5.1, 1500 6.1 and 5.6; an eighth wide:
+        // 2000 6.9 and 6.5; 1200 mixed of 0.55 to 1 times 512 KiB, whose top
+        // streams hold half the SMs, 12.7 and 10.2.
+        double free_sms = ctx->sms;
+        auto four_fits = [&](size_t wide, size_t others) {
+            return (double)wide + 0.125 * (double)others <= 3.0 * free_sms;
+        };
+        auto is_wide = [&](uint32_t i) { return ps[i].cls == kClsO1Dense && ps[i].nd > kMidMaxNd; };
+        size_t coded = 0, wide = 0;
+        for (size_t i = 0; i < nb; i++) {
+            if (ps[i].cls == kClsNone) continue;
+            if (is_top[i] && ctx->tune.o1_top_exclusive) {
+                free_sms -= is_top[i] == 1 && !is_wide((uint32_t)i) ? 1.0 / (double)top_pack : 1.0;
+            } else {
+                coded++;
+                wide += is_wide((uint32_t)i);
+            }
+        }
+        const bool four = four_fits(wide, coded - wide);
+        // Where all of them are too many but the serial-bound ones alone are
+        // not, these go there, beside the others (128 KiB full-range blocks
+        // with like-sized ones of 1 MiB: 1000 and 150 17.4 -> 10.8 ms, 500 and
+        // 250 17.1 -> 10.7).
+        if (alike && !four && ctx->tune.o1_four_max_streams < 0) {
+            std::vector<uint32_t> longest;
+            for (const auto &c : cand)
+                if (is_wide(c.second) && c.first > 0.5 * cand[0].first) longest.push_back(c.second);
+            if (four_fits(longest.size(), coded - longest.size()))
+                for (uint32_t i : longest) is_top[i] = 1;
         }
         auto group_of = [&](uint32_t i) -> int {
             const DecStream &d = ps[i];

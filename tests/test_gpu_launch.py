@@ -79,3 +79,27 @@ def test_long_wide_streams_beside_many_short_ones(codec):
     st = codec.stage_stats(True)
     assert (status == 0).all() and torch.equal(out[:len(data)], d_src)
     assert st["dec_o1_dense"]["launches"] == 1 and st["dec_o1_wide"]["launches"] == 1
+
+
+@pytest.mark.parametrize("exclusive,want", [(1, (1, 1)), (0, (2, 0))])
+def test_rule_leaves_out_the_sms_of_top_streams(codec, exclusive, want):
+    """100 top streams on SMs of their own leave room for fewer than the 150
+    others on the four-warp decoder; without SMs of their own all 250 fit."""
+    import torch
+
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("sizes are for 148 SMs")
+    rng = np.random.default_rng(2)
+    lens = np.array([60_000] * 100 + [3000] * 150, np.uint64)
+    spans = np.stack([np.concatenate([[0], np.cumsum(lens)[:-1]]).astype(np.uint64), lens], 1)
+    data = (40 + rng.integers(0, 30, int(lens.sum()))).astype(np.uint8)
+    d_src = torch.from_numpy(data).to("cuda")
+    for name, v in (("o1_four_max_streams", -1), ("o1_top_max", 111), ("o1_top_latency_pct", 75),
+                    ("o1_top_exclusive", exclusive)):
+        codec.set_param(name, v)
+    enc, streams, _ = codec.encode_batch(d_src, spans, 1)
+    codec.stage_stats(True)
+    out, _, status = codec.decode_batch(enc, streams, spans)
+    st = codec.stage_stats(True)
+    assert (status == 0).all() and torch.equal(out[:len(data)], d_src)
+    assert (st["dec_o1_dense"]["launches"], st["dec_o1_wide"]["launches"]) == want
